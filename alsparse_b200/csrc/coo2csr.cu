@@ -1,56 +1,53 @@
-// COO -> CSR on the GPU, for alphasparse_convert_csr on large COO handles.
+// COO -> CSR on the GPU, for alphasparse_convert_csr on large COO handles, and the matrices derived from a handle's
+// device copy (transpose, structured descriptors): everything that sorts stored elements.
 //
 // The reference sorts (row, column, value) records with a serial qsort and then counts rows
 // (src/core/format/convert_csr_x_coo.c:14-81); minutes at 2^28 elements.  Here the same output --
 // elements ordered by row then column, duplicates kept, in input order among equals (qsort leaves
-// that unspecified) -- comes from a stable least-significant-digit radix sort of 64-bit keys
-// (row << 32 | column) carrying the element's input position, 4 bits per pass over only the bits the
-// matrix dimensions use, followed by one binary search per row for the offsets and one gather of the
-// values.  Integer work, HBM-bound: every pass reads and writes 12 bytes per element.
+// that unspecified) -- comes from a stable least-significant-digit radix sort of keys that hold the row above
+// the column in just the bits the dimensions need (32-bit keys when they fit, else 64-bit), carrying the element's
+// position, up to 8 bits per pass, followed by one binary search per row for the offsets and one gather of the
+// values.  Integer work, HBM-bound: every pass reads the keys twice and writes keys and positions once.
 #include <algorithm>
+#include <vector>
 
 #include "internal.h"
 
 namespace asb {
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 8;  // consecutive elements per thread (blocked), so order = thread order
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kSortItems = 16;  // elements per thread, 32 apart inside the warp's run of 512: coalesced loads
 constexpr int kSortTile = kSortThreads * kSortItems;
+constexpr int kSortBins = 256;
 
+// key of a (row, column) pair: row << col_bits | column
+template <typename K>
 __global__ void coo_keys_kernel(long long nnz, const int *__restrict__ ri, const int *__restrict__ ci, int rows,
-                                int cols, unsigned long long *__restrict__ keys, unsigned *__restrict__ pos,
-                                unsigned long long *__restrict__ bad) {
+                                int cols, int col_bits, K *__restrict__ keys, unsigned long long *__restrict__ bad) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nnz) return;
     const int r = ri[i], c = ci[i];
     if (r < 0 || r >= rows || c < 0 || c >= cols) atomicAdd(bad, 1ull);
-    keys[i] = ((unsigned long long)(unsigned)r << 32) | (unsigned)c;
-    pos[i] = (unsigned)i;
+    keys[i] = ((K)(unsigned)r << col_bits) | (K)(unsigned)c;
 }
 
-// Per block: how many of its elements fall into each of the 16 digit values.  hist is digit-major
+// Per block: how many of its elements fall into each digit value.  hist is digit-major
 // (hist[d * blocks + b]) so that one exclusive scan over it yields every block's write offsets.
+template <typename K>
 __global__ void __launch_bounds__(kSortThreads)
-    radix_hist_kernel(long long n, const unsigned long long *__restrict__ keys, int shift, unsigned *__restrict__ hist) {
-    __shared__ unsigned s_cnt[16];
-    if (threadIdx.x < 16) s_cnt[threadIdx.x] = 0;
+    radix_hist_kernel(long long n, const K *__restrict__ keys, int shift, unsigned mask, unsigned *__restrict__ hist) {
+    __shared__ unsigned s_cnt[kSortBins];
+    s_cnt[threadIdx.x] = 0;
     __syncthreads();
-    const long long base = (long long)blockIdx.x * kSortTile + (long long)threadIdx.x * kSortItems;
-    unsigned local[16];
+    const long long base = (long long)blockIdx.x * kSortTile + threadIdx.x;
 #pragma unroll
-    for (int d = 0; d < 16; d++) local[d] = 0;
-#pragma unroll
-    for (int k = 0; k < kSortItems; k++)
-        if (base + k < n) {
-            const unsigned d = (unsigned)(keys[base + k] >> shift) & 15u;
-#pragma unroll
-            for (int q = 0; q < 16; q++) local[q] += (q == d);
-        }
-#pragma unroll
-    for (int d = 0; d < 16; d++)
-        if (local[d]) atomicAdd(&s_cnt[d], local[d]);
+    for (int k = 0; k < kSortItems; k++) {
+        const long long i = base + k * kSortThreads;
+        if (i < n) atomicAdd(&s_cnt[(unsigned)(keys[i] >> shift) & mask], 1u);
+    }
     __syncthreads();
-    if (threadIdx.x < 16) hist[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s_cnt[threadIdx.x];
+    hist[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = s_cnt[threadIdx.x];
 }
 
 // Exclusive scan of n unsigned values in three steps (block sums, scan of the sums by one block, add).
@@ -117,86 +114,131 @@ __global__ void __launch_bounds__(kScanThreads)
         }
 }
 
-// Stable scatter of one pass: element order inside a block is thread order then item order, so the
-// rank of an element among the block's elements with the same digit is (same-digit elements of
-// earlier threads) + (same-digit elements earlier in this thread).
+// Stable scatter of one pass.  A warp owns 512 consecutive elements and takes them 32 at a time; the lanes that hold
+// the same digit find each other with one ballot per digit bit, so an element's rank among the warp's elements of its
+// digit is (those of earlier steps) + (lower lanes of this step): element order, no atomics.  The tile is put in digit
+// order in shared memory first and then written out, so that neighbouring threads write neighbouring addresses (runs of
+// 16 elements per digit on average) where scattering straight from registers touches a sector per element: 3.7e6 64-bit
+// keys of 36 bits take 10 passes of 60 us with 4-bit digits scattered directly, 5 of 45 us this way.
+template <typename K>
 __global__ void __launch_bounds__(kSortThreads)
-    radix_scatter_kernel(long long n, const unsigned long long *__restrict__ keys_in,
-                         const unsigned *__restrict__ pos_in, int shift, const unsigned *__restrict__ offs,
-                         unsigned long long *__restrict__ keys_out, unsigned *__restrict__ pos_out) {
-    __shared__ unsigned s_cnt[16][kSortThreads + 1];
-    const int t = threadIdx.x;
-    const long long base = (long long)blockIdx.x * kSortTile + (long long)t * kSortItems;
-    unsigned long long key[kSortItems];
-    unsigned local[16];
-#pragma unroll
-    for (int d = 0; d < 16; d++) local[d] = 0;
+    radix_scatter_kernel(long long n, const K *__restrict__ keys_in, const unsigned *__restrict__ pos_in, int shift,
+                         unsigned mask, const unsigned *__restrict__ offs, K *__restrict__ keys_out,
+                         unsigned *__restrict__ pos_out) {
+    __shared__ K s_buf[kSortTile];  // the keys in digit order, then the positions
+    __shared__ unsigned s_warp[kSortWarps][kSortBins];
+    __shared__ unsigned s_dst[kSortBins];  // first destination of a digit minus its first place in the tile
+    __shared__ unsigned s_sum[kSortWarps];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const long long base = (long long)blockIdx.x * kSortTile;
+    const int count = (int)(n - base < kSortTile ? n - base : kSortTile);
+    for (int i = t; i < kSortWarps * kSortBins; i += kSortThreads) (&s_warp[0][0])[i] = 0;
+    __syncthreads();
+
+    K key[kSortItems];
+    unsigned place[kSortItems], pos[kSortItems];
+    const int first = w * (32 * kSortItems) + lane;
 #pragma unroll
     for (int k = 0; k < kSortItems; k++) {
-        key[k] = base + k < n ? keys_in[base + k] : ~0ull;
-        if (base + k < n) {
-            const unsigned d = (unsigned)(key[k] >> shift) & 15u;
-#pragma unroll
-            for (int q = 0; q < 16; q++) local[q] += (q == d);
-        }
+        const int i = first + 32 * k;
+        key[k] = i < count ? keys_in[base + i] : (K)0;
+        // no positions yet: the element's own place in the input
+        pos[k] = i < count ? (pos_in ? pos_in[base + i] : (unsigned)(base + i)) : 0u;
     }
 #pragma unroll
-    for (int d = 0; d < 16; d++) s_cnt[d][t] = local[d];
+    for (int k = 0; k < kSortItems; k++) {
+        // slots beyond the input come after every element of the tile: counted with the last digit, never written
+        const unsigned d = first + 32 * k < count ? (unsigned)(key[k] >> shift) & mask : (unsigned)kSortBins - 1;
+        unsigned peers = 0xffffffffu;
+#pragma unroll
+        for (int b = 0; b < 8; b++) {
+            const bool bit = (d >> b) & 1u;
+            const unsigned with = __ballot_sync(0xffffffffu, bit);
+            peers &= bit ? with : ~with;
+        }
+        const unsigned before = s_warp[w][d];
+        __syncwarp();
+        const unsigned lower = __popc(peers & ((1u << lane) - 1u));
+        if (lower == 0) s_warp[w][d] = before + __popc(peers);
+        place[k] = before + lower;
+        __syncwarp();
+    }
     __syncthreads();
-    // warp w turns the counts of digits 2w and 2w+1 into exclusive prefixes over the 256 threads
     {
-        const int lane = t & 31, w = t >> 5;
-        for (int d = 2 * w; d < 2 * w + 2; d++) {
-            unsigned carry = 0;
-            for (int seg = 0; seg < kSortThreads; seg += 32) {
-                const unsigned v = s_cnt[d][seg + lane];
-                unsigned inc = v;
+        // thread t is digit t: exclusive prefix of its counts over the warps, then over the digits of the tile
+        unsigned run = 0;
 #pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
-                    if (lane >= o) inc += u;
-                }
-                s_cnt[d][seg + lane] = carry + inc - v;
-                carry += __shfl_sync(0xffffffffu, inc, 31);
-            }
+        for (int v = 0; v < kSortWarps; v++) {
+            const unsigned c = s_warp[v][t];
+            s_warp[v][t] = run;
+            run += c;
+        }
+        unsigned inc = run;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned u = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += u;
+        }
+        if (lane == 31) s_sum[w] = inc;
+        __syncthreads();
+        unsigned start = inc - run;
+        for (int v = 0; v < w; v++) start += s_sum[v];
+#pragma unroll
+        for (int v = 0; v < kSortWarps; v++) s_warp[v][t] += start;
+        s_dst[t] = offs[(size_t)t * gridDim.x + blockIdx.x] - start;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < kSortItems; k++) {
+        const unsigned d = first + 32 * k < count ? (unsigned)(key[k] >> shift) & mask : (unsigned)kSortBins - 1;
+        place[k] += s_warp[w][d];
+        s_buf[place[k]] = key[k];
+    }
+    __syncthreads();
+    unsigned dst[kSortItems];
+#pragma unroll
+    for (int k = 0; k < kSortItems; k++) {
+        const int i = t + k * kSortThreads;
+        if (i < count) {
+            const K v = s_buf[i];
+            dst[k] = s_dst[(unsigned)(v >> shift) & mask] + (unsigned)i;
+            keys_out[dst[k]] = v;
         }
     }
     __syncthreads();
-    unsigned dst[16];
+    unsigned *s_pos = reinterpret_cast<unsigned *>(s_buf);
 #pragma unroll
-    for (int d = 0; d < 16; d++) dst[d] = offs[(size_t)d * gridDim.x + blockIdx.x] + s_cnt[d][t];
+    for (int k = 0; k < kSortItems; k++) s_pos[place[k]] = pos[k];
+    __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kSortItems; k++)
-        if (base + k < n) {
-            const unsigned d = (unsigned)(key[k] >> shift) & 15u;
-            unsigned where = 0;
-#pragma unroll
-            for (int q = 0; q < 16; q++)
-                if (q == d) where = dst[q]++;
-            keys_out[where] = key[k];
-            pos_out[where] = pos_in[base + k];
-        }
+    for (int k = 0; k < kSortItems; k++) {
+        const int i = t + k * kSortThreads;
+        if (i < count) pos_out[dst[k]] = s_pos[i];
+    }
 }
 
-// ptr[r] = first sorted element whose row is >= r (r = 0 .. rows); columns and values in sorted order.
-template <typename T>
-__global__ void csr_from_sorted_kernel(long long nnz, int rows, const unsigned long long *__restrict__ keys,
-                                       const unsigned *__restrict__ pos, const T *__restrict__ vals_in,
-                                       int *__restrict__ ptr, int *__restrict__ col, T *__restrict__ val) {
+// ptr[r] = first sorted element whose row is >= r (r = 0 .. rows); columns in sorted order.
+template <typename K>
+__global__ void csr_from_sorted_kernel(long long nnz, int rows, int col_bits, const K *__restrict__ keys,
+                                       int *__restrict__ ptr, int *__restrict__ col) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i <= rows) {
         long long lo = 0, hi = nnz;
         while (lo < hi) {
             const long long mid = (lo + hi) >> 1;
-            if ((long long)(keys[mid] >> 32) < i) lo = mid + 1;
+            if ((long long)(keys[mid] >> col_bits) < i) lo = mid + 1;
             else hi = mid;
         }
         ptr[i] = (int)lo;
     }
-    if (i < nnz) {
-        col[i] = (int)(unsigned)keys[i];
-        val[i] = vals_in[pos[i]];
-    }
+    if (i < nnz) col[i] = (int)(unsigned)(keys[i] & (((K)1 << col_bits) - 1));
+}
+
+template <typename T>
+__global__ void gather_values_kernel(long long nnz, const unsigned *__restrict__ pos, const T *__restrict__ in,
+                                     T *__restrict__ out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < nnz) out[i] = in[pos[i]];
 }
 
 static int bits_for(int64_t n) {
@@ -215,93 +257,128 @@ static alphasparse_status_t device_exclusive_scan(unsigned *d_data, long long n,
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
-// Host COO arrays in, HOST 3-array CSR out (caller-provided buffers of rows+1 / nnz / nnz elements).
-// All device memory is temporary.  Returns INVALID_VALUE when an index is out of range.
-template <typename T>
-alphasparse_status_t coo_to_csr_device(int64_t rows, int64_t cols, int64_t nnz, const int *ri, const int *ci,
-                                       const T *v, int *out_ptr, int *out_col, T *out_val) {
-    cudaStream_t st = current_stream();
-    const long long nblocks = (nnz + kSortTile - 1) / kSortTile;
-    const long long hist_n = 16 * nblocks;
-    const int scan_blocks = (int)((hist_n + kScanTile - 1) / kScanTile);
-    int *d_ri = nullptr, *d_ci = nullptr, *d_ptr = nullptr, *d_col = nullptr;
-    T *d_v = nullptr, *d_val = nullptr;
-    unsigned long long *d_keys[2] = {nullptr, nullptr}, *d_bad = nullptr;
-    unsigned *d_pos[2] = {nullptr, nullptr}, *d_hist = nullptr, *d_sums = nullptr;
-    alphasparse_status_t status = ALPHA_SPARSE_STATUS_SUCCESS;
-    auto release = [&]() {
-        cudaFree(d_ri), cudaFree(d_ci), cudaFree(d_ptr), cudaFree(d_col), cudaFree(d_v), cudaFree(d_val);
-        cudaFree(d_keys[0]), cudaFree(d_keys[1]), cudaFree(d_pos[0]), cudaFree(d_pos[1]);
-        cudaFree(d_hist), cudaFree(d_sums), cudaFree(d_bad);
-    };
-#define TRY(expr, code)                       \
-    do {                                      \
-        cudaError_t _e = (expr);              \
-        if (_e != cudaSuccess) {              \
-            record_cuda_error(_e, #expr);     \
-            release();                        \
-            return (code);                    \
-        }                                     \
-    } while (0)
-    const size_t n = (size_t)nnz;
-    TRY(device_alloc(&d_ri, sizeof(int) * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_ci, sizeof(int) * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_v, sizeof(T) * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_keys[0], 8 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_keys[1], 8 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_pos[0], 4 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_pos[1], 4 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_hist, sizeof(unsigned) * (size_t)hist_n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_sums, sizeof(unsigned) * (size_t)(scan_blocks + 1)), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_bad, 8), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(cudaMemsetAsync(d_bad, 0, 8, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-    TRY(cudaMemcpyAsync(d_ri, ri, sizeof(int) * n, cudaMemcpyHostToDevice, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-    TRY(cudaMemcpyAsync(d_ci, ci, sizeof(int) * n, cudaMemcpyHostToDevice, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-    TRY(cudaMemcpyAsync(d_v, v, sizeof(T) * n, cudaMemcpyHostToDevice, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+// Pieces of one device block, each on a 256-byte boundary.  First pass with a null base: how much is needed.
+struct Carve {
+    char *base;
+    size_t used = 0;
+    explicit Carve(void *p) : base(static_cast<char *>(p)) {}
+    template <typename P>
+    P *take(size_t count) {
+        char *p = base ? base + used : nullptr;
+        used += (std::max<size_t>(count, 1) * sizeof(P) + 255) & ~(size_t)255;
+        return reinterpret_cast<P *>(p);
+    }
+};
 
-    coo_keys_kernel<<<(unsigned)((nnz + 255) / 256), 256, 0, st>>>(nnz, d_ri, d_ci, (int)rows, (int)cols, d_keys[0],
-                                                                  d_pos[0], d_bad);
+// Scratch of one sort of n keys.
+template <typename K>
+struct SortScratch {
+    K *keys[2];
+    unsigned *pos[2], *hist, *sums;
+    SortScratch(Carve &c, long long n) {
+        const size_t blocks = (size_t)((n + kSortTile - 1) / kSortTile), cells = blocks * kSortBins;
+        keys[0] = c.take<K>((size_t)n), keys[1] = c.take<K>((size_t)n);
+        pos[0] = c.take<unsigned>((size_t)n), pos[1] = c.take<unsigned>((size_t)n);
+        hist = c.take<unsigned>(cells), sums = c.take<unsigned>((cells + kScanTile - 1) / kScanTile + 1);
+    }
+};
+
+// Stable sort of s.keys[0] by its low `bits` bits; `payload`: s.pos[0] holds the elements' payloads (else they are the
+// positions 0 .. n-1).  On return *cur says which of the two buffers holds the result.
+template <typename K>
+static alphasparse_status_t radix_sort(const SortScratch<K> &s, long long n, int bits, bool payload, int *cur, cudaStream_t st) {
+    const unsigned blocks = (unsigned)((n + kSortTile - 1) / kSortTile);
+    const int passes = std::max(1, (bits + 7) / 8);
+    *cur = 0;
+    for (int p = 0, shift = 0; p < passes; p++) {
+        const int width = (bits - shift + (passes - p) - 1) / (passes - p);  // the bits left, spread over the passes left
+        const unsigned mask = (1u << width) - 1u;
+        radix_hist_kernel<K><<<blocks, kSortThreads, 0, st>>>(n, s.keys[*cur], shift, mask, s.hist);
+        count_launch();
+        alphasparse_status_t status = device_exclusive_scan(s.hist, (long long)blocks * kSortBins, s.sums, st);
+        if (status != ALPHA_SPARSE_STATUS_SUCCESS) return status;
+        radix_scatter_kernel<K><<<blocks, kSortThreads, 0, st>>>(n, s.keys[*cur], p > 0 || payload ? s.pos[*cur] : nullptr, shift,
+                                                                mask, s.hist, s.keys[*cur ^ 1], s.pos[*cur ^ 1]);
+        count_launch();
+        *cur ^= 1;
+        shift += width;
+    }
+    ASB_CUDA_OR(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
+// One scratch block per conversion, given back when it goes out of scope.
+struct ScopedBlock {
+    DeviceBlock b;
+    ~ScopedBlock() { device_block_give(&b); }
+};
+
+// Host COO arrays in, device CSR (one block, ctx_adopt_block's layout) and HOST 3-array CSR out (caller-provided buffers
+// of rows+1 / nnz / nnz elements).  The index arrays go over first and are sorted while the values follow on a stream
+// of their own.  (Sending the sorted columns back while the values come in was no faster: with the cores filling and
+// emptying the rings both directions of the link slow down by what the overlap gains.)
+template <typename T, typename K>
+static alphasparse_status_t coo_to_csr_keyed(int64_t rows, int64_t cols, int64_t nnz, const int *ri, const int *ci,
+                                             const T *v, int *out_ptr, int *out_col, T *out_val, DeviceBlock *out) {
+    cudaStream_t st = current_stream();
+    ScopedBlock scratch, result;
+    const size_t n = (size_t)nnz;
+#define TRY(expr, code) ASB_CUDA_OR(expr, code)
+    auto layout = [&](void *p, int **d_ri, int **d_ci, T **d_v, unsigned long long **d_bad) {
+        Carve c(p);
+        *d_ri = c.take<int>(n), *d_ci = c.take<int>(n), *d_v = c.take<T>(n), *d_bad = c.take<unsigned long long>(1);
+        SortScratch<K> s(c, nnz);
+        return std::make_pair(s, c.used);
+    };
+    int *d_ri, *d_ci;
+    T *d_v;
+    unsigned long long *d_bad;
+    TRY(device_block_take(layout(nullptr, &d_ri, &d_ci, &d_v, &d_bad).second, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    const SortScratch<K> sort = layout(scratch.b.p, &d_ri, &d_ci, &d_v, &d_bad).first;
+    TRY(device_block_take(adopt_block_bytes(sizeof(T), rows, nnz), &result.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    int *d_ptr, *d_col;
+    T *d_val;
+    adopt_block_layout(result.b.p, rows, nnz, &d_ptr, &d_col, &d_val);
+
+    TRY(cudaMemsetAsync(d_bad, 0, 8, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    TRY(copy_to_device(d_ri, ri, sizeof(int) * n, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    TRY(copy_to_device(d_ci, ci, sizeof(int) * n, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    const unsigned blocks = (unsigned)((nnz + 255) / 256);
+    const int col_bits = bits_for(cols);
+    coo_keys_kernel<K><<<blocks, 256, 0, st>>>(nnz, d_ri, d_ci, (int)rows, (int)cols, col_bits, sort.keys[0], d_bad);
     count_launch();
     int cur = 0;
-    const int col_bits = bits_for(cols), row_bits = bits_for(rows);
-    for (int part = 0; part < 2 && status == ALPHA_SPARSE_STATUS_SUCCESS; part++) {
-        const int first = part == 0 ? 0 : 32, nbits = part == 0 ? col_bits : row_bits;
-        for (int shift = first; shift < first + nbits; shift += 4) {
-            radix_hist_kernel<<<(unsigned)nblocks, kSortThreads, 0, st>>>(nnz, d_keys[cur], shift, d_hist);
-            count_launch();
-            status = device_exclusive_scan(d_hist, hist_n, d_sums, st);
-            if (status != ALPHA_SPARSE_STATUS_SUCCESS) break;
-            radix_scatter_kernel<<<(unsigned)nblocks, kSortThreads, 0, st>>>(nnz, d_keys[cur], d_pos[cur], shift,
-                                                                            d_hist, d_keys[cur ^ 1], d_pos[cur ^ 1]);
-            count_launch();
-            cur ^= 1;
-        }
-    }
-    if (status != ALPHA_SPARSE_STATUS_SUCCESS) {
-        release();
-        return status;
-    }
-    // the input index arrays are no longer needed: reuse them for the result
-    d_ptr = nullptr;
-    TRY(device_alloc(&d_ptr, sizeof(int) * (size_t)(rows + 1)), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    TRY(device_alloc(&d_val, sizeof(T) * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-    d_col = d_ri;
-    d_ri = nullptr;
+    alphasparse_status_t status = radix_sort<K>(sort, nnz, col_bits + bits_for(rows), false, &cur, st);
+    if (status != ALPHA_SPARSE_STATUS_SUCCESS) return status;
     const long long work = std::max<long long>(nnz, rows + 1);
-    csr_from_sorted_kernel<T><<<(unsigned)((work + 255) / 256), 256, 0, st>>>(nnz, (int)rows, d_keys[cur], d_pos[cur],
-                                                                            d_v, d_ptr, d_col, d_val);
+    csr_from_sorted_kernel<K><<<(unsigned)((work + 255) / 256), 256, 0, st>>>(nnz, (int)rows, col_bits, sort.keys[cur], d_ptr,
+                                                                            d_col);
     count_launch();
-    TRY(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    TRY(cudaMemsetAsync(d_ptr + rows + 1, 0, sizeof(int) * 4, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    TRY(cudaMemsetAsync(d_col + nnz, 0, sizeof(int) * kTailPad, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    TRY(cudaMemsetAsync(d_val + nnz, 0, sizeof(T) * kTailPad, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    TRY(copy_to_device_beside(d_v, v, sizeof(T) * n, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    gather_values_kernel<T><<<blocks, 256, 0, st>>>(nnz, sort.pos[cur], d_v, d_val);
+    count_launch();
     unsigned long long bad = 0;
-    TRY(cudaMemcpyAsync(&bad, d_bad, 8, cudaMemcpyDeviceToHost, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-    TRY(cudaMemcpyAsync(out_ptr, d_ptr, sizeof(int) * (size_t)(rows + 1), cudaMemcpyDeviceToHost, st),
-        ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-    TRY(cudaMemcpyAsync(out_col, d_col, sizeof(int) * n, cudaMemcpyDeviceToHost, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-    TRY(cudaMemcpyAsync(out_val, d_val, sizeof(T) * n, cudaMemcpyDeviceToHost, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-    TRY(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-#undef TRY
-    release();
-    return bad ? ALPHA_SPARSE_STATUS_INVALID_VALUE : ALPHA_SPARSE_STATUS_SUCCESS;
+    Download back({{out_ptr, d_ptr, sizeof(int) * (size_t)(rows + 1)},
+                   {out_col, d_col, sizeof(int) * n},
+                   {out_val, d_val, sizeof(T) * n},
+                   {&bad, d_bad, 8}},
+                  st);
+    TRY(back.finish(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    if (bad) return ALPHA_SPARSE_STATUS_INVALID_VALUE;
+    *out = result.b;
+    result.b = DeviceBlock{};
+    return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
+template <typename T>
+alphasparse_status_t coo_to_csr_device(int64_t rows, int64_t cols, int64_t nnz, const int *ri, const int *ci,
+                                       const T *v, int *out_ptr, int *out_col, T *out_val, DeviceBlock *out) {
+    if (bits_for(rows) + bits_for(cols) <= 32)
+        return coo_to_csr_keyed<T, unsigned>(rows, cols, nnz, ri, ci, v, out_ptr, out_col, out_val, out);
+    return coo_to_csr_keyed<T, unsigned long long>(rows, cols, nnz, ri, ci, v, out_ptr, out_col, out_val, out);
 }
 
 // ---- A^T from the device copy of A ------------------------------------------------------------------
@@ -310,19 +387,11 @@ alphasparse_status_t coo_to_csr_device(int64_t rows, int64_t cols, int64_t nnz, 
 // and its transposed gemv adds the elements of a column of A in ascending row order
 // (src/plain/kernel/level2/mv/gemv/gemv_x_csr_trans_plain.c:14-25).  Here the same arrays come from the device copy
 // without touching the host: the stored elements, taken in storage order (rows ascending), are sorted by column
-// with the stable radix sort above (keys = column, over the bits the column count uses; the payload is the
+// with the stable radix sort above (32-bit keys = column, over the bits the column count uses; the payload is the
 // element's position), so the elements of a column come out by ascending row; the row of each is found again by a
 // binary search in the row offsets, the new offsets by a binary search in the sorted columns.
-__global__ void transpose_keys_kernel(long long nnz, const int *__restrict__ col, unsigned long long *__restrict__ keys,
-                                      unsigned *__restrict__ pos) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nnz) return;
-    keys[i] = (unsigned)col[i];
-    pos[i] = (unsigned)i;
-}
-
 template <typename T>
-__global__ void transpose_fill_kernel(long long nnz, int rows, int cols, const unsigned long long *__restrict__ keys,
+__global__ void transpose_fill_kernel(long long nnz, int rows, int cols, const unsigned *__restrict__ keys,
                                       const unsigned *__restrict__ pos, const int *__restrict__ row_ptr,
                                       const T *__restrict__ val, int *__restrict__ tptr, int *__restrict__ tcol,
                                       T *__restrict__ tval) {
@@ -331,7 +400,7 @@ __global__ void transpose_fill_kernel(long long nnz, int rows, int cols, const u
         long long lo = 0, hi = nnz;
         while (lo < hi) {
             const long long mid = (lo + hi) >> 1;
-            if ((long long)(unsigned)keys[mid] < i) lo = mid + 1;
+            if ((long long)keys[mid] < i) lo = mid + 1;
             else hi = mid;
         }
         tptr[i] = (int)lo;
@@ -355,23 +424,17 @@ template <typename T>
 alphasparse_status_t transpose_csr_device(const DeviceCtx *c, int **out_ptr, int **out_col, T **out_val) {
     cudaStream_t st = current_stream();
     const int64_t nnz = c->nnz, rows = c->rows, cols = c->cols;
-    const long long nblocks = std::max<long long>(1, (nnz + kSortTile - 1) / kSortTile);
-    const long long hist_n = 16 * nblocks;
-    const int scan_blocks = (int)((hist_n + kScanTile - 1) / kScanTile);
-    unsigned long long *d_keys[2] = {nullptr, nullptr};
-    unsigned *d_pos[2] = {nullptr, nullptr}, *d_hist = nullptr, *d_sums = nullptr;
+    ScopedBlock scratch;
     int *tptr = nullptr, *tcol = nullptr;
     T *tval = nullptr;
-    auto release = [&](bool all) {
-        cudaFree(d_keys[0]), cudaFree(d_keys[1]), cudaFree(d_pos[0]), cudaFree(d_pos[1]), cudaFree(d_hist), cudaFree(d_sums);
-        if (all) cudaFree(tptr), cudaFree(tcol), cudaFree(tval);
-    };
+    auto release = [&] { cudaFree(tptr), cudaFree(tcol), cudaFree(tval); };
+#undef TRY
 #define TRY(expr, code)                   \
     do {                                  \
         cudaError_t _e = (expr);          \
         if (_e != cudaSuccess) {          \
             record_cuda_error(_e, #expr); \
-            release(true);                \
+            release();                    \
             return (code);                \
         }                                 \
     } while (0)
@@ -383,39 +446,28 @@ alphasparse_status_t transpose_csr_device(const DeviceCtx *c, int **out_ptr, int
     TRY(cudaMemsetAsync(tcol + n, 0, sizeof(int) * kTailPad, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     TRY(cudaMemsetAsync(tval + n, 0, sizeof(T) * kTailPad, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     if (nnz > 0) {
-        TRY(device_alloc(&d_keys[0], 8 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_keys[1], 8 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_pos[0], 4 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_pos[1], 4 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_hist, sizeof(unsigned) * (size_t)hist_n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_sums, sizeof(unsigned) * (size_t)(scan_blocks + 1)), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        transpose_keys_kernel<<<(unsigned)((nnz + 255) / 256), 256, 0, st>>>(nnz, c->d_col, d_keys[0], d_pos[0]);
-        count_launch();
+        Carve need(nullptr);
+        (void)SortScratch<unsigned>(need, nnz);
+        TRY(device_block_take(need.used, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+        Carve have(scratch.b.p);
+        const SortScratch<unsigned> sort(have, nnz);
+        TRY(cudaMemcpyAsync(sort.keys[0], c->d_col, sizeof(int) * n, cudaMemcpyDeviceToDevice, st),
+            ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
         int cur = 0;
-        const int col_bits = bits_for(cols);
-        for (int shift = 0; shift < col_bits; shift += 4) {
-            radix_hist_kernel<<<(unsigned)nblocks, kSortThreads, 0, st>>>(nnz, d_keys[cur], shift, d_hist);
-            count_launch();
-            alphasparse_status_t s = device_exclusive_scan(d_hist, hist_n, d_sums, st);
-            if (s != ALPHA_SPARSE_STATUS_SUCCESS) {
-                release(true);
-                return s;
-            }
-            radix_scatter_kernel<<<(unsigned)nblocks, kSortThreads, 0, st>>>(nnz, d_keys[cur], d_pos[cur], shift, d_hist,
-                                                                            d_keys[cur ^ 1], d_pos[cur ^ 1]);
-            count_launch();
-            cur ^= 1;
+        alphasparse_status_t s = radix_sort<unsigned>(sort, nnz, bits_for(cols), false, &cur, st);
+        if (s != ALPHA_SPARSE_STATUS_SUCCESS) {
+            release();
+            return s;
         }
         const long long work = std::max<long long>(nnz, cols + 1);
         transpose_fill_kernel<T><<<(unsigned)((work + 255) / 256), 256, 0, st>>>(
-            nnz, (int)rows, (int)cols, d_keys[cur], d_pos[cur], c->d_row_ptr, static_cast<const T *>(c->d_val), tptr, tcol,
+            nnz, (int)rows, (int)cols, sort.keys[cur], sort.pos[cur], c->d_row_ptr, static_cast<const T *>(c->d_val), tptr, tcol,
             tval);
         count_launch();
         TRY(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
     TRY(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
 #undef TRY
-    release(false);
     *out_ptr = tptr, *out_col = tcol, *out_val = tval;
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
@@ -481,11 +533,11 @@ __global__ void derive_count_kernel(long long nnz, int rows, const int *__restri
 // `offset` holds the exclusive scan of the counts; the explicit unit diagonal takes the first `rows` places.
 __global__ void derive_emit_kernel(long long nnz, int rows, const int *__restrict__ row_ptr, const int *__restrict__ col,
                                    DeriveRule rule, const int *__restrict__ pick, const unsigned *__restrict__ offset,
-                                   unsigned long long *__restrict__ keys, unsigned *__restrict__ pos) {
+                                   int bits, unsigned long long *__restrict__ keys, unsigned *__restrict__ pos) {
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     const unsigned first = rule.unit ? (unsigned)rows : 0u;
     if (rule.unit && t < rows) {
-        keys[t] = ((unsigned long long)(unsigned)t << 32) | (unsigned)t;
+        keys[t] = ((unsigned long long)(unsigned)t << bits) | (unsigned)t;
         pos[t] = kUnitPayload;
     }
     if (t >= nnz) return;
@@ -494,16 +546,17 @@ __global__ void derive_emit_kernel(long long nnz, int rows, const int *__restric
     if (n == 0) return;
     const unsigned o = first + offset[k];
     const bool flip = rule.flip && j != i;
-    keys[o] = flip ? ((unsigned long long)(unsigned)j << 32) | (unsigned)i : ((unsigned long long)(unsigned)i << 32) | (unsigned)j;
+    keys[o] = flip ? ((unsigned long long)(unsigned)j << bits) | (unsigned)i
+                   : ((unsigned long long)(unsigned)i << bits) | (unsigned)j;
     pos[o] = (unsigned)k;
     if (n == 2) {
-        keys[o + 1] = ((unsigned long long)(unsigned)j << 32) | (unsigned)i;
+        keys[o + 1] = ((unsigned long long)(unsigned)j << bits) | (unsigned)i;
         pos[o + 1] = (unsigned)k;
     }
 }
 
 template <typename T>
-__global__ void derive_fill_kernel(long long m, int rows, const unsigned long long *__restrict__ keys,
+__global__ void derive_fill_kernel(long long m, int rows, int bits, const unsigned long long *__restrict__ keys,
                                    const unsigned *__restrict__ pos, const T *__restrict__ val, int *__restrict__ ptr,
                                    int *__restrict__ col_out, T *__restrict__ val_out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -511,13 +564,13 @@ __global__ void derive_fill_kernel(long long m, int rows, const unsigned long lo
         long long lo = 0, hi = m;
         while (lo < hi) {
             const long long mid = (lo + hi) >> 1;
-            if ((long long)(keys[mid] >> 32) < i) lo = mid + 1;
+            if ((long long)(keys[mid] >> bits) < i) lo = mid + 1;
             else hi = mid;
         }
         ptr[i] = (int)lo;
     }
     if (i < m) {
-        col_out[i] = (int)(unsigned)keys[i];
+        col_out[i] = (int)(unsigned)(keys[i] & ((1ull << bits) - 1));
         val_out[i] = pos[i] == kUnitPayload ? T(1) : val[pos[i]];
     }
 }
@@ -530,13 +583,12 @@ alphasparse_status_t derive_csr_device(const DeviceCtx *c, int type, int upper, 
     cudaStream_t st = current_stream();
     const int64_t nnz = c->nnz, rows = c->rows;
     const DeriveRule rule{type, upper, unit, flip, diag_rule};
-    unsigned long long *d_keys[2] = {nullptr, nullptr};
-    unsigned *d_pos[2] = {nullptr, nullptr}, *d_hist = nullptr, *d_sums = nullptr, *d_count = nullptr;
+    ScopedBlock scratch;
+    unsigned *d_sums = nullptr, *d_count = nullptr;
     int *d_pick = nullptr, *dptr = nullptr, *dcol = nullptr;
     T *dval = nullptr;
     auto release = [&](bool all) {
-        cudaFree(d_keys[0]), cudaFree(d_keys[1]), cudaFree(d_pos[0]), cudaFree(d_pos[1]), cudaFree(d_hist), cudaFree(d_sums);
-        cudaFree(d_count), cudaFree(d_pick);
+        cudaFree(d_sums), cudaFree(d_count), cudaFree(d_pick);
         if (all) cudaFree(dptr), cudaFree(dcol), cudaFree(dval);
     };
 #define TRY(expr, code)                   \
@@ -593,40 +645,25 @@ alphasparse_status_t derive_csr_device(const DeviceCtx *c, int type, int upper, 
     TRY(cudaMemsetAsync(dcol + n, 0, sizeof(int) * kTailPad, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     TRY(cudaMemsetAsync(dval + n, 0, sizeof(T) * kTailPad, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     if (m > 0) {
-        const long long nblocks = (m + kSortTile - 1) / kSortTile;
-        const long long hist_n = 16 * nblocks;
-        const int scan_blocks = (int)((hist_n + kScanTile - 1) / kScanTile);
-        TRY(device_alloc(&d_keys[0], 8 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_keys[1], 8 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_pos[0], 4 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_pos[1], 4 * n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_hist, sizeof(unsigned) * (size_t)hist_n), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        TRY(device_alloc(&d_sums, sizeof(unsigned) * (size_t)(scan_blocks + 1)), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+        Carve need(nullptr);
+        (void)SortScratch<unsigned long long>(need, m);
+        TRY(device_block_take(need.used, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+        Carve have(scratch.b.p);
+        const SortScratch<unsigned long long> sort(have, m);
+        const int bits = bits_for(rows);  // square: rows == cols
         const long long work = std::max<long long>(nnz, unit ? rows : 0);
         derive_emit_kernel<<<(unsigned)((work + 255) / 256), 256, 0, st>>>(nnz, (int)rows, c->d_row_ptr, c->d_col, rule,
-                                                                          d_pick, d_count, d_keys[0], d_pos[0]);
+                                                                          d_pick, d_count, bits, sort.keys[0], sort.pos[0]);
         count_launch();
         int cur = 0;
-        const int bits = bits_for(rows);  // square: rows == cols
-        for (int part = 0; part < 2; part++) {
-            const int first = part == 0 ? 0 : 32;
-            for (int shift = first; shift < first + bits; shift += 4) {
-                radix_hist_kernel<<<(unsigned)nblocks, kSortThreads, 0, st>>>(m, d_keys[cur], shift, d_hist);
-                count_launch();
-                alphasparse_status_t s = device_exclusive_scan(d_hist, hist_n, d_sums, st);
-                if (s != ALPHA_SPARSE_STATUS_SUCCESS) {
-                    release(true);
-                    return s;
-                }
-                radix_scatter_kernel<<<(unsigned)nblocks, kSortThreads, 0, st>>>(m, d_keys[cur], d_pos[cur], shift, d_hist,
-                                                                                d_keys[cur ^ 1], d_pos[cur ^ 1]);
-                count_launch();
-                cur ^= 1;
-            }
+        alphasparse_status_t s = radix_sort<unsigned long long>(sort, m, 2 * bits, true, &cur, st);
+        if (s != ALPHA_SPARSE_STATUS_SUCCESS) {
+            release(true);
+            return s;
         }
         const long long fill = std::max<long long>(m, rows + 1);
         derive_fill_kernel<T><<<(unsigned)((fill + 255) / 256), 256, 0, st>>>(
-            m, (int)rows, d_keys[cur], d_pos[cur], static_cast<const T *>(c->d_val), dptr, dcol, dval);
+            m, (int)rows, bits, sort.keys[cur], sort.pos[cur], static_cast<const T *>(c->d_val), dptr, dcol, dval);
         count_launch();
         TRY(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
@@ -646,8 +683,8 @@ template alphasparse_status_t transpose_csr_device<float>(const DeviceCtx *, int
 template alphasparse_status_t transpose_csr_device<double>(const DeviceCtx *, int **, int **, double **);
 
 template alphasparse_status_t coo_to_csr_device<float>(int64_t, int64_t, int64_t, const int *, const int *,
-                                                       const float *, int *, int *, float *);
+                                                       const float *, int *, int *, float *, DeviceBlock *);
 template alphasparse_status_t coo_to_csr_device<double>(int64_t, int64_t, int64_t, const int *, const int *,
-                                                        const double *, int *, int *, double *);
+                                                        const double *, int *, int *, double *, DeviceBlock *);
 
 }  // namespace asb

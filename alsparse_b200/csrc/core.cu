@@ -46,15 +46,24 @@ alphasparse_cuda_alg_t forced_algorithm() {
 
 static std::atomic<long long> g_fail_alloc_in{0};  // > 0: that many allocations from now, the last one fails
 
-cudaError_t device_alloc_bytes(void **p, size_t bytes) {
+bool device_alloc_denied() {
     long long left = g_fail_alloc_in.load(std::memory_order_relaxed);
     while (left > 0 && !g_fail_alloc_in.compare_exchange_weak(left, left - 1)) {
     }
-    if (left == 1) {
+    return left == 1;
+}
+
+cudaError_t device_alloc_bytes(void **p, size_t bytes) {
+    if (device_alloc_denied()) {
         *p = nullptr;
         return cudaErrorMemoryAllocation;
     }
-    return cudaMalloc(p, bytes);
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && device_cache_trim()) {
+        (void)cudaGetLastError();
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
 }
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
@@ -126,9 +135,14 @@ void ctx_destroy(DeviceCtx *c) {
     int prev = -1;
     cudaGetDevice(&prev);
     cudaSetDevice(c->device);
-    cudaFree(c->d_row_ptr);
-    cudaFree(c->d_col);
-    cudaFree(c->d_val);
+    if (c->block.p) {
+        device_block_give(&c->block);
+    } else {
+        cudaFree(c->d_row_ptr);
+        cudaFree(c->d_col);
+        cudaFree(c->d_val);
+        cudaFree(c->d_status);
+    }
     cudaFree(c->d_tile);
     cudaFree(c->d_carry_row);
     cudaFree(c->d_carry_val);
@@ -143,7 +157,6 @@ void ctx_destroy(DeviceCtx *c) {
     cudaFree(c->d_cm_y);
     cudaFree(c->d_x_stage);
     cudaFree(c->d_y_stage);
-    cudaFree(c->d_status);
     if (c->copy_in) cudaStreamDestroy(c->copy_in);
     if (c->copy_out) cudaStreamDestroy(c->copy_out);
     for (cudaEvent_t ev : c->ev_pipe)
@@ -193,17 +206,13 @@ alphasparse_status_t ctx_create(int datatype, int64_t rows, int64_t cols, const 
     c->device_bytes = (int64_t)(sizeof(int) * (size_t)(rows + 1) + (sizeof(int) + tsz) * padded);
 
     if (rows > 0) {
-        TRY(cudaMemcpyAsync(c->d_row_ptr, ptr, sizeof(int) * (size_t)(rows + 1),
-                            cudaMemcpyHostToDevice, st),
-            ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+        TRY(copy_to_device(c->d_row_ptr, ptr, sizeof(int) * (size_t)(rows + 1), st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     } else {
         TRY(cudaMemsetAsync(c->d_row_ptr, 0, sizeof(int), st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
     if (c->nnz > 0) {
-        TRY(cudaMemcpyAsync(c->d_col, col, sizeof(int) * (size_t)c->nnz, cudaMemcpyHostToDevice, st),
-            ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-        TRY(cudaMemcpyAsync(c->d_val, val, tsz * (size_t)c->nnz, cudaMemcpyHostToDevice, st),
-            ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+        TRY(copy_to_device(c->d_col, col, sizeof(int) * (size_t)c->nnz, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+        TRY(copy_to_device(c->d_val, val, tsz * (size_t)c->nnz, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
     TRY(cudaMemsetAsync(c->d_col + c->nnz, 0, sizeof(int) * kTailPad, st),
         ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
@@ -250,6 +259,62 @@ alphasparse_status_t ctx_adopt(int datatype, int64_t rows, int64_t cols, int64_t
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
+// Layout of a recycled block: offsets, columns and values as ctx_create lays them out, the error word and the counters.
+struct BlockLayout {
+    size_t col, val, status, stats, bytes;
+    BlockLayout(size_t tsz, int64_t rows, int64_t nnz) {
+        auto up = [](size_t b) { return (b + 255) & ~(size_t)255; };
+        col = up(sizeof(int) * (size_t)(rows + 1 + 4));
+        val = col + up(sizeof(int) * ((size_t)nnz + kTailPad));
+        status = val + up(tsz * ((size_t)nnz + kTailPad));
+        stats = status + 256;
+        bytes = stats + 256;
+    }
+};
+size_t adopt_block_bytes(size_t tsz, int64_t rows, int64_t nnz) { return BlockLayout(tsz, rows, nnz).bytes; }
+template <typename T>
+void adopt_block_layout(void *block, int64_t rows, int64_t nnz, int **d_ptr, int **d_col, T **d_val) {
+    const BlockLayout l(sizeof(T), rows, nnz);
+    char *p = static_cast<char *>(block);
+    *d_ptr = reinterpret_cast<int *>(p), *d_col = reinterpret_cast<int *>(p + l.col), *d_val = reinterpret_cast<T *>(p + l.val);
+}
+template void adopt_block_layout<float>(void *, int64_t, int64_t, int **, int **, float **);
+template void adopt_block_layout<double>(void *, int64_t, int64_t, int **, int **, double **);
+
+alphasparse_status_t ctx_adopt_block(int datatype, int64_t rows, int64_t cols, int64_t nnz, DeviceBlock *block,
+                                     const int *h_ptr, DeviceCtx **out) {
+    *out = nullptr;
+    DeviceCtx *c = new (std::nothrow) DeviceCtx();
+    if (!c) {
+        device_block_give(block);
+        return ALPHA_SPARSE_STATUS_ALLOC_FAILED;
+    }
+    const size_t tsz = datatype == ALPHA_SPARSE_DATATYPE_DOUBLE ? 8 : 4;
+    const BlockLayout l(tsz, rows, nnz);
+    char *p = static_cast<char *>(block->p);
+    c->block = *block;
+    *block = DeviceBlock{};
+    c->device = c->block.device, c->datatype = datatype, c->rows = rows, c->cols = cols, c->nnz = nnz;
+    c->d_row_ptr = reinterpret_cast<int *>(p), c->d_col = reinterpret_cast<int *>(p + l.col), c->d_val = p + l.val;
+    c->d_status = reinterpret_cast<int *>(p + l.status), c->d_stats = reinterpret_cast<unsigned long long *>(p + l.stats);
+    c->device_bytes = (int64_t)l.bytes;
+    cudaError_t e = cudaMemsetAsync(c->d_status, 0, sizeof(int), current_stream());
+    alphasparse_status_t s = ALPHA_SPARSE_STATUS_EXECUTION_FAILED;
+    if (e == cudaSuccess) {
+        c->h_row_ptr = h_ptr;
+        s = ctx_analyse(c);
+        c->h_row_ptr = nullptr;
+    } else {
+        record_cuda_error(e, "ctx_adopt_block");
+    }
+    if (s != ALPHA_SPARSE_STATUS_SUCCESS) {
+        ctx_destroy(c);
+        return s;
+    }
+    *out = c;
+    return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
 // ---- host copies ---------------------------------------------------------------------------------
 
 template <typename T>
@@ -268,12 +333,6 @@ struct CsrOf<double> {
     using csc = spmat_csc_d_t;
     static constexpr alphasparse_datatype_t dt = ALPHA_SPARSE_DATATYPE_DOUBLE;
 };
-
-static void *host_alloc(size_t bytes) {
-    void *p = nullptr;
-    if (posix_memalign(&p, 64, bytes ? bytes : 64) != 0) return nullptr;
-    return p;
-}
 
 template <typename T>
 static void free_csr_host(typename CsrOf<T>::csr *m) {
@@ -311,15 +370,17 @@ static RegistryEntry registry_take(const void *record) {
 }
 
 // Takes ownership of ptr / col / val (host_alloc'ed, zero-based 3-array CSR) and builds the
-// handle around them: host record for export_csr, device copy and analysis for mv / mm.
+// handle around them: host record for export_csr, device copy (or the block that already holds the same arrays) and
+// analysis for mv / mm.
 template <typename T>
 static alphasparse_status_t finish_csr_handle(alphasparse_matrix_t *A, int64_t rows, int64_t cols,
-                                              int *ptr, int *col, T *val) {
+                                              int *ptr, int *col, T *val, DeviceBlock *on_device = nullptr) {
     using M = typename CsrOf<T>::csr;
     alphasparse_matrix *h = static_cast<alphasparse_matrix *>(calloc(1, sizeof(alphasparse_matrix)));
     M *m = static_cast<M *>(calloc(1, sizeof(M)));
     if (!h || !m) {
         free(h), free(m), free(ptr), free(col), free(val);
+        if (on_device) device_block_give(on_device);
         return ALPHA_SPARSE_STATUS_ALLOC_FAILED;
     }
     m->values = val;
@@ -334,7 +395,8 @@ static alphasparse_status_t finish_csr_handle(alphasparse_matrix_t *A, int64_t r
     h->datatype = CsrOf<T>::dt;
 
     DeviceCtx *c = nullptr;
-    alphasparse_status_t s = ctx_create(CsrOf<T>::dt, rows, cols, ptr, col, val, &c);
+    alphasparse_status_t s = on_device ? ctx_adopt_block(CsrOf<T>::dt, rows, cols, ptr[rows], on_device, ptr, &c)
+                                       : ctx_create(CsrOf<T>::dt, rows, cols, ptr, col, val, &c);
     if (s != ALPHA_SPARSE_STATUS_SUCCESS) {
         free_csr_host<T>(m);
         free(h);
@@ -380,11 +442,13 @@ static alphasparse_status_t create_csr(alphasparse_matrix_t *A, alphasparse_inde
     ptr[0] = 0;
 #pragma omp parallel for schedule(static) if (rows > (1 << 16))
     for (int64_t i = 0; i < rows; i++) ptr[i + 1] = rows_end[i] - first;
+    if (shift == 0) {
+        host_copy(col, col_indx, sizeof(int) * (size_t)nnz);
+    } else {
 #pragma omp parallel for schedule(static) if (nnz > (1 << 16))
-    for (int64_t i = 0; i < nnz; i++) {
-        col[i] = col_indx[i] - shift;
-        val[i] = values[i];
+        for (int64_t i = 0; i < nnz; i++) col[i] = col_indx[i] - shift;
     }
+    host_copy(val, values, sizeof(T) * (size_t)nnz);
     return finish_csr_handle<T>(A, rows, cols, ptr, col, val);
 }
 
@@ -452,12 +516,17 @@ static alphasparse_status_t create_coo(alphasparse_matrix_t *A, alphasparse_inde
         free(h), free(m), free(ri), free(ci), free(v);
         return ALPHA_SPARSE_STATUS_ALLOC_FAILED;
     }
+    if (shift == 0) {
+        host_copy(ri, row_indx, sizeof(int) * (size_t)nnz);
+        host_copy(ci, col_indx, sizeof(int) * (size_t)nnz);
+    } else {
 #pragma omp parallel for schedule(static) if (nnz > (1 << 16))
-    for (int64_t i = 0; i < nnz; i++) {
-        ri[i] = row_indx[i] - shift;
-        ci[i] = col_indx[i] - shift;
-        v[i] = values[i];
+        for (int64_t i = 0; i < nnz; i++) {
+            ri[i] = row_indx[i] - shift;
+            ci[i] = col_indx[i] - shift;
+        }
     }
+    host_copy(v, values, sizeof(T) * (size_t)nnz);
     m->values = v, m->row_indx = ri, m->col_indx = ci;
     m->rows = rows, m->cols = cols, m->nnz = nnz, m->ordered = false;
     h->mat = m;
@@ -514,6 +583,10 @@ static alphasparse_status_t triples_to_csr(int64_t rows, int64_t nnz, const int 
 // Equal (row, column) pairs keep their input order (qsort leaves theirs unspecified).
 // With transpose = true rows and columns swap roles (the reference transposes the COO handle
 // first, src/core/op_/alphasparse_convert_csr.c:144-151).
+// From this many elements on the sort runs on the GPU (coo2csr.cu).  Handle from triples on the B200 host, fp64,
+// 7,500 / 15,000 / 60,000 / 960,000 / 3,750,000 elements: 0.32 / 0.52 / 1.17 / 14.2 / 62 ms on the host path,
+// 0.26 / 0.28 / 0.41 / 1.27 / 6.4 ms here.
+constexpr int64_t kDeviceSortMin = 1 << 13;
 template <typename T>
 static alphasparse_status_t coo_to_csr(const typename CsrOf<T>::coo *src, bool transpose,
                                        alphasparse_matrix_t *dest) {
@@ -522,12 +595,12 @@ static alphasparse_status_t coo_to_csr(const typename CsrOf<T>::coo *src, bool t
     const int64_t nnz = src->nnz;
     const int *ri = transpose ? src->col_indx : src->row_indx;
     const int *ci = transpose ? src->row_indx : src->col_indx;
-    // Large inputs are sorted on the GPU (radix sort, coo2csr.cu); ALPHASPARSE_CUDA_COO=host|device forces a path.
+    // ALPHASPARSE_CUDA_COO=host|device forces a path.
     static const int forced = [] {
         const char *e = getenv("ALPHASPARSE_CUDA_COO");
         return !e ? 0 : !strcmp(e, "host") ? 1 : !strcmp(e, "device") ? 2 : 0;
     }();
-    if (nnz > 0 && forced != 1 && (forced == 2 || nnz >= (1 << 20))) {
+    if (nnz > 0 && forced != 1 && (forced == 2 || nnz >= kDeviceSortMin)) {
         int *ptr = static_cast<int *>(host_alloc(sizeof(int) * (size_t)(rows + 1)));
         int *col = static_cast<int *>(host_alloc(sizeof(int) * (size_t)nnz));
         T *val = static_cast<T *>(host_alloc(sizeof(T) * (size_t)nnz));
@@ -535,12 +608,13 @@ static alphasparse_status_t coo_to_csr(const typename CsrOf<T>::coo *src, bool t
             free(ptr), free(col), free(val);
             return ALPHA_SPARSE_STATUS_ALLOC_FAILED;
         }
-        alphasparse_status_t s = coo_to_csr_device<T>(rows, cols, nnz, ri, ci, src->values, ptr, col, val);
+        DeviceBlock block;
+        alphasparse_status_t s = coo_to_csr_device<T>(rows, cols, nnz, ri, ci, src->values, ptr, col, val, &block);
         if (s != ALPHA_SPARSE_STATUS_SUCCESS) {
             free(ptr), free(col), free(val);
             return s;
         }
-        return finish_csr_handle<T>(dest, rows, cols, ptr, col, val);
+        return finish_csr_handle<T>(dest, rows, cols, ptr, col, val, &block);
     }
     for (int64_t i = 0; i < nnz; i++)
         if (ri[i] < 0 || ri[i] >= rows || ci[i] < 0 || ci[i] >= cols)

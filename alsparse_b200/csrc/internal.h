@@ -6,6 +6,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <initializer_list>
 #include <mutex>
 #include <vector>
 
@@ -55,6 +56,49 @@ enum Option {
     kOptCount
 };
 int64_t option(Option o);
+
+// ---- memory and copies of handle creation (transfer.cu) ------------------------------------
+void *host_alloc(size_t bytes);  // released with free(); large arrays on 2 MB pages
+void host_copy(void *dst, const void *src, size_t bytes);  // memcpy, by several threads when large
+// Host -> device on the current device, ordered on `st`.  Returns when a pageable `src` may be reused.
+cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st);
+// ... on a stream of its own, beside what is queued on `st` (which must not touch `dst`); later work on `st` waits for it.
+cudaError_t copy_to_device_beside(void *dst, const void *src, size_t bytes, cudaStream_t st);
+// Device -> host, any number of arrays one behind the other: the constructor enqueues what fits the page-locked ring
+// behind the work on `st`, finish() moves the rest and returns when every destination is complete.  Downloads of one
+// device run one after the other (a live object holds the ring), so a thread has at most one at a time.
+struct Ring;
+class Download {
+  public:
+    struct Piece {
+        void *dst;
+        const void *src;
+        size_t bytes;
+    };
+    Download(std::initializer_list<Piece> pieces, cudaStream_t st);
+    ~Download();
+    Download(const Download &) = delete;
+    Download &operator=(const Download &) = delete;
+    cudaError_t finish();
+
+  private:
+    void issue();
+    std::vector<Piece> chunks_;
+    size_t issued_ = 0, done_ = 0;
+    cudaStream_t st_;
+    Ring *ring_ = nullptr;
+    cudaError_t error_ = cudaSuccess;
+};
+// Device memory of conversions, recycled through a small bounded cache.
+struct DeviceBlock {
+    void *p = nullptr;
+    size_t bytes = 0;
+    int device = 0;
+};
+cudaError_t device_block_take(size_t bytes, DeviceBlock *out);
+void device_block_give(DeviceBlock *b);  // waits until the device is idle
+bool device_cache_trim();                // gives everything cached back to CUDA; true if there was anything
+bool device_alloc_denied();              // counts an allocation for alphasparse_cuda_debug_fail_alloc; true: it is to fail
 
 // Every device allocation of the library goes through here: cudaMalloc, except that a test can ask
 // for the n-th allocation from now on to fail (alphasparse_cuda_debug_fail_alloc), which is how the
@@ -227,6 +271,8 @@ struct DeviceCtx {
     BandTables band;                   // long rows taken out of the merge tiles (spmv_band.cu); rows == 0: none
     unsigned *d_chunk_done = nullptr;  // per chunk of kPushChunkTiles tiles (exchange calls only)
 
+    DeviceBlock block;                       // holds d_row_ptr .. d_val, d_status and d_stats when it is set
+    unsigned long long *d_stats = nullptr;  // counters of the analysis (kept: allocations are what creation waits for)
     int *d_status = nullptr;  // error word set by kernels whose bounded waits ran out (0 = fine)
 
     // staging for calls that pass host vectors (grown on demand, reused)
@@ -262,6 +308,12 @@ alphasparse_status_t ctx_create(int datatype, int64_t rows, int64_t cols, const 
 // and values with zeroed tails) and analyses them.  Takes the arrays over: on failure they are freed.
 alphasparse_status_t ctx_adopt(int datatype, int64_t rows, int64_t cols, int64_t nnz, int *d_ptr, int *d_col,
                                void *d_val, DeviceCtx **out);
+// The same for arrays in one recycled block (adopt_block_layout); `h_ptr`: the offsets on the host.
+size_t adopt_block_bytes(size_t tsz, int64_t rows, int64_t nnz);
+template <typename T>
+void adopt_block_layout(void *block, int64_t rows, int64_t nnz, int **d_ptr, int **d_col, T **d_val);
+alphasparse_status_t ctx_adopt_block(int datatype, int64_t rows, int64_t cols, int64_t nnz, DeviceBlock *block,
+                                     const int *h_ptr, DeviceCtx **out);
 void ctx_destroy(DeviceCtx *ctx);
 alphasparse_status_t ctx_analyse(DeviceCtx *ctx);
 
@@ -321,9 +373,10 @@ alphasparse_status_t derive_csr_device(const DeviceCtx *c, int type, int upper, 
                                        int **out_ptr, int **out_col, T **out_val, int64_t *out_nnz);
 
 // COO -> CSR on the device (coo2csr.cu): host arrays in, host 3-array CSR out, same output as the host
-// path in core.cu (ordered by row then column, equal pairs in input order).
+// path in core.cu (ordered by row then column, equal pairs in input order), and the same arrays on the device in a
+// block for ctx_adopt_block.
 template <typename T>
 alphasparse_status_t coo_to_csr_device(int64_t rows, int64_t cols, int64_t nnz, const int *ri, const int *ci,
-                                       const T *v, int *out_ptr, int *out_col, T *out_val);
+                                       const T *v, int *out_ptr, int *out_col, T *out_val, DeviceBlock *out);
 
 }  // namespace asb

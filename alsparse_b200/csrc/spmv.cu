@@ -919,8 +919,8 @@ alphasparse_status_t ctx_analyse(DeviceCtx *ctx) {
     ctx->max_row_nnz = 0, ctx->empty_rows = ctx->rows, ctx->mean_row_nnz = 0.0;
     if (ctx->rows == 0) return ALPHA_SPARSE_STATUS_SUCCESS;
 
-    unsigned long long *d_out = nullptr, h_out[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    ASB_CUDA_OR(device_alloc(&d_out, sizeof(h_out)), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    unsigned long long *d_out = ctx->d_stats, h_out[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    if (!d_out) ASB_CUDA_OR(device_alloc(&d_out, sizeof(h_out)), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
     cudaError_t e = cudaMemsetAsync(d_out, 0, sizeof(h_out), st);
     if (e == cudaSuccess) {
         const int threads = 256;
@@ -943,7 +943,7 @@ alphasparse_status_t ctx_analyse(DeviceCtx *ctx) {
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(h_out, d_out, sizeof(h_out), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d_out);
+    if (!ctx->d_stats) cudaFree(d_out);
     if (e != cudaSuccess) {
         record_cuda_error(e, "row analysis");
         return ALPHA_SPARSE_STATUS_EXECUTION_FAILED;

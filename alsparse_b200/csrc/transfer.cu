@@ -1,0 +1,325 @@
+// Memory and copies of handle creation: large host arrays on 2 MB pages, copies between pageable host memory and the
+// device through page-locked rings filled by all cores, and a small cache of device blocks for matrices that are
+// assembled again and again.
+//
+// Measured on the B200 host (16 cores): a pageable cudaMemcpy moves 11-18 GB/s, single-threaded, and a fresh host array
+// costs 1.1 us per 4 KB page on top (9 ms for 32 MB, 29 ms for 64 MB).  Four 4 MB page-locked chunks filled by OpenMP
+// threads while the copy engine drains the others reach 40-44 GB/s of the 53 GB/s the link gives page-locked memory
+// (chunks of 1 / 2 / 4 / 8 MB: 29 / 36 / 44 / 41 GB/s), and 2 MB pages bring the first touch of 64 MB from 2.5 to 1.3 ms
+// with every core, 29 to 13 ms with one.  cudaMalloc and cudaFree take 0.3-3 ms each there.
+#include <emmintrin.h>
+#include <stdlib.h>
+#include <string.h>
+#include <sys/mman.h>
+
+#include <omp.h>
+
+#include <algorithm>
+#include <mutex>
+#include <vector>
+
+#include "internal.h"
+
+namespace asb {
+
+constexpr size_t kHugePage = (size_t)2 << 20;
+
+// Arrays of 32 MB and more are always mapped afresh by malloc: on 2 MB pages, with every page touched once by all cores
+// (a 4 MB piece of an untouched array takes 350-500 us to copy into, however many threads share its two pages, 4 MB of
+// touched memory 80 us).  Smaller arrays come from malloc as they are: it recycles them, and keeping them here instead
+// made the caller's own arrays of the same sizes slower.
+constexpr size_t kMappedBytes = (size_t)32 << 20;
+
+void *host_alloc(size_t bytes) {
+    void *p = nullptr;
+    const bool huge = bytes >= kMappedBytes;
+    if (posix_memalign(&p, huge ? kHugePage : 64, bytes ? bytes : 64) != 0) return nullptr;
+    if (huge) {
+        (void)madvise(p, bytes & ~(kHugePage - 1), MADV_HUGEPAGE);  // advice: where it is refused, small pages serve
+        char *c = static_cast<char *>(p);
+#pragma omp parallel for schedule(static)
+        for (int64_t i = 0; i < (int64_t)(bytes >> 12); i++) c[i << 12] = 0;
+    }
+    return p;
+}
+
+// Copies past the caches: the destination is read next by the copy engine, or much later.  (What a core leaves dirty in
+// its cache the copy engine has to fetch from there: the last chunks of an upload, read after the cores had gone idle,
+// took 250-420 us per 4 MB instead of 80.)
+static void copy_streaming(char *dst, const char *src, size_t bytes) {
+    const size_t head = std::min<size_t>(bytes, (16 - (reinterpret_cast<uintptr_t>(dst) & 15)) & 15);
+    memcpy(dst, src, head);
+    dst += head, src += head, bytes -= head;
+    for (; bytes >= 64; bytes -= 64, dst += 64, src += 64) {
+        const __m128i *s = reinterpret_cast<const __m128i *>(src);
+        __m128i *d = reinterpret_cast<__m128i *>(dst);
+        const __m128i a = _mm_loadu_si128(s), b = _mm_loadu_si128(s + 1), c = _mm_loadu_si128(s + 2), e = _mm_loadu_si128(s + 3);
+        _mm_stream_si128(d, a), _mm_stream_si128(d + 1, b), _mm_stream_si128(d + 2, c), _mm_stream_si128(d + 3, e);
+    }
+    memcpy(dst, src, bytes);
+    _mm_sfence();
+}
+
+// memcpy by all cores once the piece is worth waking them for
+void host_copy(void *dst, const void *src, size_t bytes) {
+    constexpr size_t kPerThread = 128 << 10;
+    const int threads = (int)std::min<size_t>((size_t)std::max(1, omp_get_max_threads()), bytes / kPerThread);
+    if (threads <= 1) {
+        memcpy(dst, src, bytes);
+        return;
+    }
+#pragma omp parallel num_threads(threads)
+    {
+        const size_t t = (size_t)omp_get_thread_num(), nt = (size_t)omp_get_num_threads();
+        const size_t a = (bytes * t / nt) & ~(size_t)63, e = t + 1 == nt ? bytes : (bytes * (t + 1) / nt) & ~(size_t)63;
+        copy_streaming(static_cast<char *>(dst) + a, static_cast<const char *>(src) + a, e - a);
+    }
+}
+
+// ---- page-locked rings ------------------------------------------------------------------------------
+//
+// One ring per direction and device, made on first use and kept (2 x 16 MB page-locked per device in use).  A transfer
+// holds its ring's lock; an upload returns once its last piece is in the ring (the source may go away), a download
+// once everything is in host memory.
+
+constexpr int kRingChunks = 4;
+constexpr size_t kRingChunkBytes = (size_t)4 << 20;
+constexpr size_t kRingMinBytes = 64 << 10;  // below this one pageable cudaMemcpyAsync is as fast
+constexpr int kRingDevices = 64;
+
+struct Ring {
+    std::mutex mu;
+    bool ready = false;
+    char *buf[kRingChunks] = {};
+    cudaEvent_t ev[kRingChunks] = {};
+    int next = 0;
+    cudaStream_t side = nullptr;  // copy_to_device_beside
+    cudaEvent_t side_done = nullptr;
+};
+static Ring g_up[kRingDevices], g_down[kRingDevices];
+
+static cudaError_t ring_of_current_device(Ring *rings, Ring **out) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    *out = nullptr;
+    if (e == cudaSuccess && dev < kRingDevices) *out = &rings[dev];
+    return e;
+}
+
+// with the ring's lock held; a ring that cannot be made stays unready and the caller copies directly
+static bool ring_ready(Ring &r) {
+    if (r.ready) return true;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < kRingChunks && e == cudaSuccess; k++) {
+        if (!r.buf[k]) e = cudaHostAlloc(reinterpret_cast<void **>(&r.buf[k]), kRingChunkBytes, cudaHostAllocDefault);
+        if (e == cudaSuccess && !r.ev[k]) e = cudaEventCreateWithFlags(&r.ev[k], cudaEventDisableTiming);
+    }
+    if (e != cudaSuccess) (void)cudaGetLastError();
+    return r.ready = e == cudaSuccess;
+}
+
+static bool page_locked(const void *p) {
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return at.type != cudaMemoryTypeUnregistered;
+}
+
+cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    if (bytes == 0) return cudaSuccess;
+    Ring *ring = nullptr;
+    if (bytes >= kRingMinBytes && !page_locked(src)) {
+        cudaError_t e = ring_of_current_device(g_up, &ring);
+        if (e != cudaSuccess) return e;
+    }
+    if (!ring) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    std::lock_guard<std::mutex> lock(ring->mu);
+    if (!ring_ready(*ring)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    for (size_t off = 0; off < bytes; off += kRingChunkBytes) {
+        const size_t n = std::min(kRingChunkBytes, bytes - off);
+        const int k = ring->next;
+        ring->next = (k + 1) % kRingChunks;
+        cudaError_t e = cudaEventSynchronize(ring->ev[k]);  // the copy that used this chunk last is done
+        if (e != cudaSuccess) return e;
+        host_copy(ring->buf[k], static_cast<const char *>(src) + off, n);
+        e = cudaMemcpyAsync(static_cast<char *>(dst) + off, ring->buf[k], n, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaEventRecord(ring->ev[k], st);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+cudaError_t copy_to_device_beside(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    Ring *ring = nullptr;
+    cudaError_t e = ring_of_current_device(g_up, &ring);
+    if (e != cudaSuccess) return e;
+    if (!ring || bytes < kRingMinBytes) return copy_to_device(dst, src, bytes, st);
+    cudaStream_t side = nullptr;
+    cudaEvent_t done = nullptr;
+    {
+        std::lock_guard<std::mutex> lock(ring->mu);
+        if (!ring->side_done) {
+            e = cudaStreamCreateWithFlags(&ring->side, cudaStreamNonBlocking);
+            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ring->side_done, cudaEventDisableTiming);
+            if (e != cudaSuccess) return e;
+        }
+        side = ring->side, done = ring->side_done;
+    }
+    e = copy_to_device(dst, src, bytes, side);
+    // (two threads may record one after the other: both copies are then in front of the later record, and the earlier
+    // waiter waits for at least its own)
+    if (e == cudaSuccess) e = cudaEventRecord(done, side);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(st, done, 0);
+    return e;
+}
+
+Download::Download(std::initializer_list<Piece> pieces, cudaStream_t st) : st_(st) {
+    size_t total = 0;
+    for (const Piece &p : pieces) {
+        total += p.bytes;
+        for (size_t off = 0; off < p.bytes; off += kRingChunkBytes)
+            chunks_.push_back({static_cast<char *>(p.dst) + off, static_cast<const char *>(p.src) + off,
+                               std::min(kRingChunkBytes, p.bytes - off)});
+    }
+    if (total < kRingMinBytes) return;  // copied by finish()
+    Ring *ring = nullptr;
+    error_ = ring_of_current_device(g_down, &ring);
+    if (error_ != cudaSuccess || !ring) return;
+    ring->mu.lock();
+    if (!ring_ready(*ring)) {
+        ring->mu.unlock();
+        return;
+    }
+    ring_ = ring;
+    while (issued_ < chunks_.size() && issued_ < kRingChunks && error_ == cudaSuccess) issue();
+}
+
+void Download::issue() {
+    const Piece &c = chunks_[issued_];
+    const size_t k = issued_ % kRingChunks;
+    error_ = cudaMemcpyAsync(ring_->buf[k], c.src, c.bytes, cudaMemcpyDeviceToHost, st_);
+    if (error_ == cudaSuccess) error_ = cudaEventRecord(ring_->ev[k], st_);
+    issued_++;
+}
+
+cudaError_t Download::finish() {
+    for (; done_ < chunks_.size() && error_ == cudaSuccess; done_++) {
+        const Piece &c = chunks_[done_];
+        if (!ring_) {
+            error_ = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, st_);
+            continue;
+        }
+        const size_t k = done_ % kRingChunks;
+        error_ = cudaEventSynchronize(ring_->ev[k]);
+        if (error_ != cudaSuccess) break;
+        host_copy(c.dst, ring_->buf[k], c.bytes);
+        if (issued_ < chunks_.size()) issue();
+    }
+    if (!ring_ && error_ == cudaSuccess) error_ = cudaStreamSynchronize(st_);
+    return error_;
+}
+
+Download::~Download() {
+    if (!ring_) return;
+    if (done_ < issued_) (void)cudaStreamSynchronize(st_);  // given up half-way: nothing may still write into the ring
+    ring_->mu.unlock();
+}
+
+// ---- device blocks of assembled matrices ---------------------------------------------------------------
+//
+// Converting triples needs scratch for the sort and one block for the resulting arrays.  A program that assembles its
+// matrix at every step would pay cudaMalloc and cudaFree for both each time (1-6 ms of a 5 ms conversion), so blocks
+// given back here are kept for the next conversion: at most kCacheBytes over all devices, the oldest leave first, and
+// all of them when an allocation fails.  A block is idle when it enters (the giver waits for the device, as cudaFree
+// does), so it can be used on any stream by any thread.
+
+constexpr size_t kCacheBytes = (size_t)512 << 20;
+constexpr size_t kCacheGrain = (size_t)256 << 10;
+
+struct CacheBlock {
+    void *p;
+    size_t bytes;
+    int device;
+};
+static std::mutex g_cache_mu;
+static std::vector<CacheBlock> g_cache;  // oldest first
+
+static void cache_free(const CacheBlock &b) {
+    int prev = -1;
+    cudaGetDevice(&prev);
+    if (prev != b.device) cudaSetDevice(b.device);
+    cudaFree(b.p);
+    if (prev >= 0 && prev != b.device) cudaSetDevice(prev);
+}
+
+bool device_cache_trim() {
+    std::vector<CacheBlock> out;
+    {
+        std::lock_guard<std::mutex> lock(g_cache_mu);
+        out.swap(g_cache);
+    }
+    for (const CacheBlock &b : out) cache_free(b);
+    return !out.empty();
+}
+
+cudaError_t device_block_take(size_t bytes, DeviceBlock *out) {
+    *out = DeviceBlock{};
+    const size_t want = (std::max<size_t>(bytes, 1) + kCacheGrain - 1) / kCacheGrain * kCacheGrain;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (device_alloc_denied()) return cudaErrorMemoryAllocation;
+    {
+        std::lock_guard<std::mutex> lock(g_cache_mu);
+        size_t best = g_cache.size();
+        for (size_t i = 0; i < g_cache.size(); i++)
+            if (g_cache[i].device == dev && g_cache[i].bytes >= want && g_cache[i].bytes <= 2 * want &&
+                (best == g_cache.size() || g_cache[i].bytes < g_cache[best].bytes))
+                best = i;
+        if (best < g_cache.size()) {
+            out->p = g_cache[best].p, out->bytes = g_cache[best].bytes, out->device = dev;
+            g_cache.erase(g_cache.begin() + (ptrdiff_t)best);
+            return cudaSuccess;
+        }
+    }
+    e = cudaMalloc(&out->p, want);
+    if (e == cudaErrorMemoryAllocation && device_cache_trim()) {
+        (void)cudaGetLastError();
+        e = cudaMalloc(&out->p, want);
+    }
+    if (e == cudaSuccess) out->bytes = want, out->device = dev;
+    return e;
+}
+
+void device_block_give(DeviceBlock *b) {
+    if (!b->p) return;
+    const CacheBlock mine{b->p, b->bytes, b->device};
+    *b = DeviceBlock{};
+    if (mine.bytes > kCacheBytes / 2) {
+        cache_free(mine);
+        return;
+    }
+    int prev = -1;
+    cudaGetDevice(&prev);
+    if (prev != mine.device) cudaSetDevice(mine.device);
+    const cudaError_t e = cudaDeviceSynchronize();
+    if (prev >= 0 && prev != mine.device) cudaSetDevice(prev);
+    std::vector<CacheBlock> out;
+    {
+        std::lock_guard<std::mutex> lock(g_cache_mu);
+        if (e == cudaSuccess) g_cache.push_back(mine);
+        else out.push_back(mine);
+        size_t total = 0;
+        for (const CacheBlock &c : g_cache) total += c.bytes;
+        while (total > kCacheBytes) {
+            total -= g_cache.front().bytes;
+            out.push_back(g_cache.front());
+            g_cache.erase(g_cache.begin());
+        }
+    }
+    for (const CacheBlock &c : out) cache_free(c);
+}
+
+}  // namespace asb
