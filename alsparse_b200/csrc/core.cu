@@ -152,6 +152,7 @@ void ctx_destroy(DeviceCtx *c) {
     bins_destroy(c->bins);
     spmm_blocks_destroy(c->spmm);
     spmm_split_destroy(c->split);
+    spmm_segments_destroy(c->segments);
     spmm_blocks_destroy(c->mvb);
     cudaFree(c->d_cm_x);
     cudaFree(c->d_cm_y);

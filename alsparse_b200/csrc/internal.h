@@ -215,7 +215,7 @@ struct DeviceCtx;
 // b.blocks == 1 when the rows are not in ascending column order.
 alphasparse_status_t col_blocks_ensure(DeviceCtx *ctx, SpmmBlocks &b, int blocks, cudaStream_t st);
 
-// Long rows of the row-major dense-block product (spmm.cu).  One lane group per row is fine until a row holds a
+// Long rows of the narrow and the column-major dense-block product (spmm.cu).  One lane group per row is fine until a row holds a
 // hundred thousand elements and its group is still walking it long after every other row is done: rows above
 // `spmm_split_min` elements are left out of the row pass (their end in d_hi_short is their start), cut into chunks of
 // `spmm_split_chunk` elements that the same kernel multiplies as if they were rows, into partial sums, and a last
@@ -231,6 +231,20 @@ struct SpmmSplit {
     size_t part_bytes = 0;
 };
 void spmm_split_destroy(SpmmSplit &s);
+
+// Segments of the row-major dense-block product on a matrix with uneven rows (spmm_stream_kernel).
+struct SpmmSegments {
+    int state = 0;  // 0: not looked at yet, 1: even rows, no table, 2: tables below are in use
+    int nseg = 0;
+    int64_t nslots = 0;                          // segments that leave a part of a row behind
+    MergeCoord *d_seg = nullptr;                 // nseg + 1 starts
+    int *d_slot = nullptr;                       // nseg: place of what the segment leaves behind, or -1
+    int *d_row = nullptr, *d_first = nullptr;    // rows cut over segments, and the first slot of each (one more closes)
+    std::vector<int> seg_row, cross_row, cross_first;  // host copies: what a row window owns
+    void *d_part = nullptr;                      // nslots x columns partial sums
+    size_t part_bytes = 0;
+};
+void spmm_segments_destroy(SpmmSegments &s);
 
 struct DeviceCtx {
     uint64_t magic = kCtxMagic;
@@ -263,7 +277,8 @@ struct DeviceCtx {
     RowBins bins;                      // row bins of a skewed matrix; active: products run bin by bin
     const int *h_row_ptr = nullptr;    // host copy of the offsets, valid only while the handle is being created
     SpmmBlocks spmm;                   // column blocks of the row-major dense-block product
-    SpmmSplit split;                   // its long rows, cut into chunks
+    SpmmSegments segments;             // its segments when rows are uneven
+    SpmmSplit split;                   // long rows of the narrow and the column-major product, cut into chunks
     void *d_cm_x = nullptr, *d_cm_y = nullptr;  // row-major copies of column-major dense operands (spmm.cu), grown on demand
     size_t cm_x_bytes = 0, cm_y_bytes = 0;
     SpmmBlocks mvb;                    // column blocks of the vector-kernel SpMV, for an x that does not fit L2

@@ -6,14 +6,16 @@
 // element before the accumulation).  The reference's own device build has no row-major SpMM
 // (src/kernel/dcu/level3/mm/csrmm/dcu_gemm_x_csr_row.cpp:15-36 returns NOT_SUPPORTED).
 //
-// One warp owns one sparse row; its lanes span the dense columns, VEC consecutive columns
-// per lane, so every stored element turns into one fully coalesced read of a row of X
-// (64 fp32 columns = 256 bytes = 32 lanes x float2).  The warp fetches 32 (col, alpha*a)
-// pairs with one coalesced load each and hands them round with shuffles; the loop over the
-// 32 pairs is unrolled so several X rows are in flight per warp.  Bandwidth-bound: the
+// A group of lanes spans the dense columns, VEC consecutive columns per lane, so every stored element
+// turns into one fully coalesced read of a row of X (64 fp32 columns = 256 bytes = 16 lanes x
+// float4).  The group fetches (col, alpha*a) pairs with coalesced loads and hands them round with
+// shuffles; several X rows are in flight per group.  Bandwidth-bound: the
 // traffic is nnz * columns * sizeof(T) of X rows against 2 flops per element, far below what
 // would justify staging tiles for tensor cores.
+#include <limits.h>
+
 #include <algorithm>
+#include <vector>
 
 #include "internal.h"
 
@@ -124,6 +126,232 @@ __global__ void __launch_bounds__(256, kSpmmMinBlocks)
 #pragma unroll
             for (int i = 0; i < VEC; i++) ps[i] = acc[i];
             __stcs(reinterpret_cast<P *>(out), packed);
+        }
+    }
+}
+
+// ---- the stream kernel ---------------------------------------------------------------------------------
+//
+// What bounds this product is the stream of X rows into the SMs: L2 delivers it at 19-20 TB/s (rows of 128 bytes and
+// more; 64-byte rows 17 TB/s, one request per SM and clock below that) when enough loads are in flight, HBM random
+// 256-byte rows at 7-10.  The kernel above has 4 rows in flight per lane group, none while a group fetches its next
+// elements or offsets, and issues everything once per group.  Here a warp walks a contiguous SEGMENT of the stored
+// elements, row boundaries or not: LPR lanes per X row, so 32 / LPR consecutive elements per step; the X rows of the next
+// U steps are requested before those of the current U are multiplied, elements are fetched two batches ahead and the
+// ends of the next 32 rows wait in registers.  A row that ends is summed over the lane groups and written at once; what a
+// segment holds of a row that goes on behind its end is left in `part` for spmm_cross_reduce_kernel.
+//
+// Measured (B200, us, kernel above -> here): 2^20 rows of 32 elements x 64 fp32 columns 1720 -> 1200 (X = 268 MB), 2^18
+// rows 308 -> 193 (11 TB/s), 300,007 rows of 27 x 16 columns 130 -> 92, power-law 400,009 rows x 24 columns 627 -> 188,
+// 20,000 rows x 12 columns 423 -> 14.  U = 4 with 3 or 4 blocks per SM: 1270-1335 / 212-245; U = 2 with 5 or 6 blocks
+// (spills): 1320-1430.  One segment per lane group instead of per warp: 1660-1900, the groups of a warp run apart.
+//
+// Segments: `per_warp` whole rows each (even matrices, no table), or the table of spmm_segments_ensure (skewed ones).
+constexpr int kStreamUnroll = 2;     // steps per group; two groups are in flight
+constexpr int kStreamMinBlocks = 4;  // 64 registers
+struct StreamSegments {
+    const MergeCoord *seg;  // nseg + 1 starts (null: per_warp rows each)
+    const int *slot;        // place in `part` of what a segment leaves unfinished
+    int nseg;
+    int per_warp;
+    int row0, row1;  // the rows to produce (a window of the matrix)
+};
+
+template <typename T, int VEC, int LPR, bool HAS_BETA>
+__global__ void __launch_bounds__(256, kStreamMinBlocks)
+    spmm_stream_kernel(const StreamSegments sg, const int *__restrict__ row_ptr, const int *__restrict__ col,
+                       const T *__restrict__ val, const T *__restrict__ X, int columns, int ldx, T *__restrict__ Y,
+                       long long ldy, T *__restrict__ part, T alpha, T beta) {
+    constexpr int U = kStreamUnroll;
+    constexpr int S = 32 / LPR;                        // elements per step
+    constexpr int Q = LPR < 2 * U ? 2 * U / LPR : 1;  // elements a lane holds of one batch
+    constexpr int G = LPR * Q / U;                     // groups of U steps per batch: even, for the two buffers
+    static_assert(G % 2 == 0, "groups alternate between two buffers");
+    const int lane = threadIdx.x & 31, gl = lane % LPR, sub = lane / LPR;
+    const int g = blockIdx.x * 8 + (threadIdx.x >> 5);
+    int r, r_end, k, k_end, slot = -1;
+    if (sg.seg) {
+        if (g >= sg.nseg) return;
+        const MergeCoord a = sg.seg[g], b = sg.seg[g + 1];
+        r = a.row, k = a.nz, r_end = b.row, k_end = b.nz;
+        slot = __ldg(sg.slot + g);
+        if (r < sg.row0) r = sg.row0, k = __ldg(row_ptr + r);
+        if (r_end >= sg.row1) r_end = sg.row1, k_end = __ldg(row_ptr + r_end), slot = -1;
+    } else {
+        const long long first = sg.row0 + (long long)g * sg.per_warp;
+        if (first >= sg.row1) return;
+        r = (int)first, r_end = (int)min((long long)sg.row1, first + sg.per_warp);
+        k = __ldg(row_ptr + r), k_end = __ldg(row_ptr + r_end);
+    }
+    const int c = blockIdx.y * (LPR * VEC) + gl * VEC;
+    const bool live = c < columns;
+    const T *Xc = X + (live ? c : 0);  // (lanes beyond the last column read the first and drop it)
+
+    // ends of rows r .. r + 31 (lane by lane), and of the 32 rows behind them
+    auto load_ends = [&](int from) { return from + lane < r_end ? __ldg(row_ptr + from + lane + 1) : INT_MAX; };
+    int ends = load_ends(r), ends_next = load_ends(r + 32), at = 0;
+    // Elements of this batch, the next and the one behind it.  Beyond the segment: column 0, which is read and dropped.
+    int cj[Q], cn[Q], cm[Q];
+    T vj[Q], vn[Q], vm[Q];
+    auto load_batch = [&](int from, int (&cc)[Q], T (&vv)[Q]) {
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const int j = from + q * 32 + lane;
+            cc[q] = 0, vv[q] = T(0);
+            if (j < k_end) cc[q] = __ldcs(col + j), vv[q] = __ldcs(val + j);
+        }
+    };
+    load_batch(k, cj, vj);
+    load_batch(k + 32 * Q, cn, vn);
+    T xv[2][U][VEC];
+    auto load_rows = [&](int buf, int group, const int (&cc)[Q]) {  // X rows of the U steps of a group
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int e = (group * U + u) * S;
+            const int j = __shfl_sync(0xffffffffu, cc[e / 32], e % 32 + sub);
+            load_vec<T, VEC>(Xc + (size_t)(unsigned)j * (unsigned)ldx, xv[buf][u]);
+        }
+    };
+    T acc[VEC], old[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; i++) acc[i] = T(0), old[i] = T(0);
+    using P = typename Pack<T, VEC>::type;
+    auto fetch_old = [&] {  // Y of the row in work, long before it is needed
+        if (HAS_BETA && live && sub == 0 && r < r_end) {
+            const P t = __ldcs(reinterpret_cast<const P *>(Y + r * ldy + c));
+            const T *ts = reinterpret_cast<const T *>(&t);
+#pragma unroll
+            for (int i = 0; i < VEC; i++) old[i] = ts[i];
+        }
+    };
+    fetch_old();
+    int row_end = __shfl_sync(0xffffffffu, ends, 0);
+    auto sum_groups = [&] {
+#pragma unroll
+        for (int o = LPR; o < 32; o <<= 1)
+#pragma unroll
+            for (int i = 0; i < VEC; i++) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], o);
+    };
+    auto finish_row = [&] {
+        sum_groups();
+        P packed;
+        T *ps = reinterpret_cast<T *>(&packed);
+#pragma unroll
+        for (int i = 0; i < VEC; i++) {
+            ps[i] = HAS_BETA ? fma(beta, old[i], acc[i]) : acc[i];
+            acc[i] = T(0);
+        }
+        if (live && sub == 0) __stcs(reinterpret_cast<P *>(Y + r * ldy + c), packed);
+        r++;
+        if (++at == 32) {
+            at = 0, ends = ends_next;
+            ends_next = load_ends(r + 32);
+        }
+        row_end = __shfl_sync(0xffffffffu, ends, at);
+        fetch_old();
+    };
+    while (row_end == k) finish_row();  // empty rows
+    if (k < k_end) load_rows(0, 0, cj);
+    while (k < k_end) {  // (everything about k is uniform over the warp)
+        const int k0 = k;
+        load_batch(k0 + 64 * Q, cm, vm);
+#pragma unroll
+        for (int q = 0; q < Q; q++) vj[q] *= alpha;
+#pragma unroll
+        for (int grp = 0; grp < G; grp++) {
+            if (grp + 1 < G) load_rows((grp + 1) & 1, grp + 1, cj);
+            else load_rows(0, 0, cn);
+            const int kg = k0 + grp * (U * S);
+            if (kg + U * S <= min(row_end, k_end)) {
+#pragma unroll
+                for (int u = 0; u < U; u++) {
+                    const int e = (grp * U + u) * S;
+                    const T a = __shfl_sync(0xffffffffu, vj[e / 32], e % 32 + sub);
+#pragma unroll
+                    for (int i = 0; i < VEC; i++) acc[i] = fma(a, xv[grp & 1][u][i], acc[i]);
+                }
+                k = kg + U * S;
+                while (row_end == k) finish_row();
+            } else {  // row by row through the group
+                const int stop = min(kg + U * S, k_end);
+                while (k < stop) {
+                    const int hi = min(row_end, stop);
+#pragma unroll
+                    for (int u = 0; u < U; u++) {
+                        const int e = (grp * U + u) * S;
+                        const T a = __shfl_sync(0xffffffffu, vj[e / 32], e % 32 + sub);
+                        if (k0 + e + sub >= k && k0 + e + sub < hi) {
+#pragma unroll
+                            for (int i = 0; i < VEC; i++) acc[i] = fma(a, xv[grp & 1][u][i], acc[i]);
+                        }
+                    }
+                    k = hi;
+                    while (row_end == k) finish_row();
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < Q; q++) cj[q] = cn[q], vj[q] = vn[q], cn[q] = cm[q], vn[q] = vm[q];
+    }
+    if (slot >= 0) {
+        sum_groups();
+        P packed;
+        T *ps = reinterpret_cast<T *>(&packed);
+#pragma unroll
+        for (int i = 0; i < VEC; i++) ps[i] = acc[i];
+        if (live && sub == 0) *reinterpret_cast<P *>(part + (size_t)slot * columns + c) = packed;
+    }
+}
+
+// Start of every segment: the point on the diagonal i * items of the walk through elements and row ends in which a row
+// end counts as kStreamRowItems elements (finishing a row costs a group about as much as loading that many).  A start
+// inside a row of at most kStreamWhole elements moves back to the row's beginning: short rows are never cut.
+constexpr int kStreamRowItems = 8, kStreamWhole = 64;
+__global__ void spmm_segments_kernel(int rows, int nnz, const int *__restrict__ row_ptr, int items, int nseg,
+                                     MergeCoord *__restrict__ out, int *__restrict__ slot) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > nseg) return;
+    const long long diag = (long long)i * items;
+    int lo = 0, hi = rows;  // rows whose end lies at or before the diagonal
+    while (lo < hi) {
+        const int mid = lo + ((hi - lo) >> 1);
+        if ((long long)row_ptr[mid + 1] + (long long)kStreamRowItems * (mid + 1) <= diag) lo = mid + 1;
+        else hi = mid;
+    }
+    int nz = nnz;
+    bool cut = false;
+    if (lo < rows) {
+        const int s = row_ptr[lo], e = row_ptr[lo + 1];
+        const long long at = diag - (long long)kStreamRowItems * lo;
+        nz = e - s <= kStreamWhole || at < s ? s : at > e ? e : (int)at;
+        cut = nz > s;
+    }
+    out[i].row = lo, out[i].nz = nz;
+    if (i > 0) slot[i - 1] = cut ? 0 : -1;  // the segment before leaves a part of row lo behind
+}
+
+// Y[row, :] += what the segments before the row's last one hold of it, in order.  One block per such row: the threads
+// span the columns; with few columns several runs of segments are summed side by side and then added up in order.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    spmm_cross_reduce_kernel(const int *__restrict__ row_of, const int *__restrict__ first_of, const T *__restrict__ part,
+                             int columns, T *__restrict__ Y, long long ldy) {
+    __shared__ T s_sum[256];
+    const int row = row_of[blockIdx.x], k0 = first_of[blockIdx.x], k1 = first_of[blockIdx.x + 1];
+    const int wide = min(columns, (int)blockDim.x), runs = blockDim.x / wide;
+    const int run = threadIdx.x / wide, lane = threadIdx.x % wide;
+    const int per = (k1 - k0 + runs - 1) / runs;
+    for (int c0 = 0; c0 < columns; c0 += wide) {
+        const int c = c0 + lane;
+        T acc = T(0);
+        if (run < runs && c < columns)
+            for (int k = k0 + run * per, e = min(k1, k + per); k < e; k++) acc += part[(size_t)k * columns + c];
+        __syncthreads();
+        s_sum[threadIdx.x] = acc;
+        __syncthreads();
+        if (run == 0 && c < columns) {
+            for (int v = 1; v < runs; v++) acc += s_sum[v * wide + lane];
+            Y[(long long)row * ldy + c] += acc;
         }
     }
 }
@@ -389,6 +617,100 @@ static alphasparse_status_t spmm_split_prepare(DeviceCtx *ctx, size_t tsz, int c
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
+// ---- segments of a skewed matrix ---------------------------------------------------------------------
+
+void spmm_segments_destroy(SpmmSegments &s) {
+    cudaFree(s.d_seg), cudaFree(s.d_slot), cudaFree(s.d_row), cudaFree(s.d_first), cudaFree(s.d_part);
+    s = SpmmSegments{};
+}
+
+// Built at the first product of a handle whose rows are uneven (the rule of spmm_split_ensure: even rows need no table).
+// Segments of 64 to 256 items, enough of them to keep every warp of the chip (about 5,000) busy twice.
+static alphasparse_status_t spmm_segments_ensure(DeviceCtx *ctx, cudaStream_t st) {
+    SpmmSegments &sp = ctx->segments;
+    if (sp.state != 0) return ALPHA_SPARSE_STATUS_SUCCESS;
+    const int64_t most = std::max<int64_t>(64, std::min<int64_t>(256, option(kOptSpmmSplitChunk)));
+    if (option(kOptSpmmSplitMin) <= 0 || ctx->max_row_nnz <= kStreamWhole || (double)ctx->max_row_nnz <= 8.0 * ctx->mean_row_nnz) {
+        sp.state = 1;
+        return ALPHA_SPARSE_STATUS_SUCCESS;
+    }
+    const int64_t total = ctx->nnz + kStreamRowItems * ctx->rows;
+    int64_t items = 64;
+    while (items < most && total / items > 2 * 5000) items *= 2;
+    items = std::min(items, most);
+    SpmmSegments t;
+    t.nseg = (int)((total + items - 1) / items);
+    auto fail = [&](alphasparse_status_t s) {
+        spmm_segments_destroy(t);
+        return s;
+    };
+    std::vector<int> slot, first;
+    std::vector<MergeCoord> seg;
+    cudaError_t e = device_alloc(&t.d_seg, sizeof(MergeCoord) * ((size_t)t.nseg + 1));
+    if (e == cudaSuccess) e = device_alloc(&t.d_slot, sizeof(int) * (size_t)t.nseg);
+    if (e != cudaSuccess) {
+        record_cuda_error(e, "segments of the dense-block product");
+        return fail(ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    }
+    spmm_segments_kernel<<<(unsigned)(t.nseg / 256 + 1), 256, 0, st>>>((int)ctx->rows, (int)ctx->nnz, ctx->d_row_ptr, (int)items,
+                                                                      t.nseg, t.d_seg, t.d_slot);
+    count_launch();
+    try {
+        seg.resize((size_t)t.nseg + 1), slot.resize((size_t)t.nseg);
+        e = cudaMemcpyAsync(seg.data(), t.d_seg, sizeof(MergeCoord) * seg.size(), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(slot.data(), t.d_slot, sizeof(int) * slot.size(), cudaMemcpyDeviceToHost, st);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+        if (e == cudaSuccess) {
+            t.seg_row.resize(seg.size());
+            for (size_t i = 0; i < seg.size(); i++) t.seg_row[i] = seg[i].row;
+            for (size_t i = 0; i < slot.size(); i++) {
+                if (slot[i] < 0) continue;
+                const int row = seg[i + 1].row;  // slots of a row are neighbours: its segments are
+                if (t.cross_row.empty() || t.cross_row.back() != row) t.cross_row.push_back(row), t.cross_first.push_back((int)t.nslots);
+                slot[i] = (int)t.nslots++;
+            }
+            t.cross_first.push_back((int)t.nslots);
+        }
+    } catch (...) {
+        return fail(ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    }
+    const size_t ncross = t.cross_row.size();
+    if (e == cudaSuccess && ncross > 0) {
+        e = device_alloc(&t.d_row, sizeof(int) * ncross);
+        if (e == cudaSuccess) e = device_alloc(&t.d_first, sizeof(int) * (ncross + 1));
+        if (e == cudaSuccess) e = cudaMemcpyAsync(t.d_row, t.cross_row.data(), sizeof(int) * ncross, cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess)
+            e = cudaMemcpyAsync(t.d_first, t.cross_first.data(), sizeof(int) * (ncross + 1), cudaMemcpyHostToDevice, st);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(t.d_slot, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice, st);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (e != cudaSuccess) {
+        record_cuda_error(e, "segments of the dense-block product");
+        return fail(e == cudaErrorMemoryAllocation ? ALPHA_SPARSE_STATUS_ALLOC_FAILED : ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    }
+    t.state = 2;
+    sp = t;
+    ctx->device_bytes += (int64_t)(12 * (size_t)t.nseg + 8 * ncross);
+    return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
+// The table (first product of the handle) and room for the partial sums of a product with `columns` columns.
+static alphasparse_status_t spmm_segments_prepare(DeviceCtx *ctx, size_t tsz, int columns, cudaStream_t st) {
+    alphasparse_status_t s = spmm_segments_ensure(ctx, st);
+    SpmmSegments &sp = ctx->segments;
+    if (s != ALPHA_SPARSE_STATUS_SUCCESS || sp.state != 2) return s;
+    const size_t want = tsz * (size_t)sp.nslots * (size_t)columns;
+    if (sp.part_bytes < want) {
+        cudaFree(sp.d_part);
+        ctx->device_bytes -= (int64_t)sp.part_bytes;
+        sp.d_part = nullptr, sp.part_bytes = 0;
+        ASB_CUDA_OR(device_alloc(&sp.d_part, want), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+        sp.part_bytes = want;
+        ctx->device_bytes += (int64_t)want;
+    }
+    return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
 // Column blocks are used only when asked for (option spmm_col_blocks > 1).  Measured on B200 with 64 fp32 columns,
 // 2^21 rows of 32 elements and a 537 MB X: 3.51 ms in one pass, 4.08 / 4.60 / 5.16 / 6.37 ms with 4 / 6 / 8 / 12
 // blocks.  Blocking does take the reads of X off HBM, but every stored element still pulls a whole row of X from
@@ -399,24 +721,19 @@ static int spmm_pick_blocks(const DeviceCtx *, size_t) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(blocks, 64));
 }
 
+// One pass per column block (option spmm_col_blocks): spmm_row_kernel over the part of every row inside the block.
 template <typename T, int VEC, int LPR>
-static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
-                       int ldy, cudaStream_t st, const RowWindow *w) {
+static void launch_row_blocks(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
+                              int ldy, cudaStream_t st, const RowWindow *w) {
     constexpr int rows_per_block = 8 * (32 / LPR);
     // A window is the same kernel on a slice: offsets are absolute, so shifting the offset arrays and Y
     // by the first row is all it takes.
     const int64_t first = w ? w->begin : 0, rows = w ? w->count : ctx->rows;
     const unsigned blocks = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
     const T *val = static_cast<const T *>(ctx->d_val);
-    T *const Y0 = Y;
     Y += first * (int64_t)ldy;
-    const SpmmSplit &sp = ctx->split;
-    const bool split = sp.state == 2;
-    const int passes = !split && ctx->spmm.d_split ? ctx->spmm.blocks : 1;
-    if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
-    for (int p = 0; p < passes; p++) {
-        const int *lo = passes > 1 ? ctx->spmm.d_split + (size_t)p * ctx->rows + first : ctx->d_row_ptr + first;
-        const int *hi = passes > 1 ? lo + ctx->rows : split ? sp.d_hi_short + first : lo + 1;
+    for (int p = 0; p < ctx->spmm.blocks; p++) {
+        const int *lo = ctx->spmm.d_split + (size_t)p * ctx->rows + first, *hi = lo + ctx->rows;
         // the first pass applies beta, the later ones add to what is there
         const T b = p == 0 ? beta : T(1);
         if (b == T(0))
@@ -426,35 +743,65 @@ static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx
             spmm_row_kernel<T, VEC, LPR, true><<<blocks, 256, 0, st>>>(
                 (int)rows, lo, hi, ctx->d_col, val, X, columns, ldx, Y, ldy, alpha, b);
     }
-    if (split) {
-        // the long rows of this window: their chunks through the same kernel into partial sums, then onto Y
-        const int *lb = std::lower_bound(sp.h_long_row, sp.h_long_row + sp.nlong, (int)first);
-        const int *le = std::lower_bound(sp.h_long_row, sp.h_long_row + sp.nlong, (int)(first + rows));
-        const int64_t l0 = lb - sp.h_long_row, l1 = le - sp.h_long_row;
-        const int64_t c0 = sp.h_long_first[l0], c1 = sp.h_long_first[l1];
-        if (c1 > c0) {
-            T *part = static_cast<T *>(sp.d_part) + (size_t)c0 * columns;
-            const unsigned cblocks = (unsigned)((c1 - c0 + rows_per_block - 1) / rows_per_block);
-            spmm_row_kernel<T, VEC, LPR, false><<<cblocks, 256, 0, st>>>(
-                (int)(c1 - c0), sp.d_chunk_lo + c0, sp.d_chunk_hi + c0, ctx->d_col, val, X, columns, ldx, part, columns, alpha,
-                T(0));
-            const int threads = std::min(256, (columns + 31) / 32 * 32);
-            spmm_long_reduce_kernel<T><<<(unsigned)(l1 - l0), threads, 0, st>>>(
-                sp.d_long_row + l0, sp.d_long_first + l0, static_cast<const T *>(sp.d_part), columns, Y0, ldy);
-            count_launch(2);
+    count_launch(ctx->spmm.blocks);
+}
+
+template <typename T, int VEC, int LPR>
+static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
+                       int ldy, cudaStream_t st, const RowWindow *w) {
+    SpmmSegments &sp = ctx->segments;
+    if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
+    if (sp.state != 2 && ctx->spmm.d_split) {
+        launch_row_blocks<T, VEC, LPR>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+        if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
+        return;
+    }
+    const int row0 = (int)(w ? w->begin : 0), row1 = (int)(w ? w->begin + w->count : ctx->rows);
+    StreamSegments sg{};
+    sg.row0 = row0, sg.row1 = row1;
+    int64_t groups;
+    if (sp.state == 2) {
+        // segments that hold anything of the window: the first one that ends at or behind its first row, up to the
+        // first one that ends at or behind its end
+        const auto b = sp.seg_row.begin() + 1, e = sp.seg_row.end();
+        const int64_t s0 = std::lower_bound(b, e, row0) - b, s1 = std::min<int64_t>(sp.nseg, std::lower_bound(b, e, row1) - b + 1);
+        sg.seg = sp.d_seg + s0, sg.slot = sp.d_slot + s0, sg.nseg = (int)(s1 - s0);
+        groups = s1 - s0;
+    } else {
+        // whole rows, about 256 elements a warp, but no fewer warps than the chip holds twice
+        const int64_t rows = row1 - row0, resident = 148ll * 4 * 8;
+        int64_t per = (int64_t)(256.0 / std::max(1.0, ctx->mean_row_nnz));
+        per = std::max<int64_t>(1, std::min<int64_t>(std::min<int64_t>(per, 64), rows / (2 * resident)));
+        sg.per_warp = (int)per;
+        groups = (rows + per - 1) / per;
+    }
+    const T *val = static_cast<const T *>(ctx->d_val);
+    T *part = static_cast<T *>(sp.d_part);
+    const dim3 grid((unsigned)((groups + 7) / 8), (unsigned)((columns + LPR * VEC - 1) / (LPR * VEC)));
+    if (beta == T(0))
+        spmm_stream_kernel<T, VEC, LPR, false><<<grid, 256, 0, st>>>(sg, ctx->d_row_ptr, ctx->d_col, val, X, columns, ldx, Y, ldy,
+                                                                    part, alpha, beta);
+    else
+        spmm_stream_kernel<T, VEC, LPR, true><<<grid, 256, 0, st>>>(sg, ctx->d_row_ptr, ctx->d_col, val, X, columns, ldx, Y, ldy,
+                                                                   part, alpha, beta);
+    count_launch();
+    if (sp.state == 2) {
+        const int64_t l0 = std::lower_bound(sp.cross_row.begin(), sp.cross_row.end(), row0) - sp.cross_row.begin();
+        const int64_t l1 = std::lower_bound(sp.cross_row.begin(), sp.cross_row.end(), row1) - sp.cross_row.begin();
+        if (l1 > l0) {
+            spmm_cross_reduce_kernel<T><<<(unsigned)(l1 - l0), 256, 0, st>>>(sp.d_row + l0, sp.d_first + l0, part, columns, Y, ldy);
+            count_launch();
         }
     }
     if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
-    count_launch(passes);
 }
 
 template <typename T, int VEC>
 static void launch_row_lanes(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
                              int ldy, cudaStream_t st, const RowWindow *w) {
-    // smallest group (2 .. 32 lanes) whose lanes cover the dense columns in one pass, if any
+    // smallest group (4 .. 32 lanes) whose lanes cover the dense columns in one pass, if any
     const int need = (columns + VEC - 1) / VEC;
-    if (need <= 2) launch_row<T, VEC, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
-    else if (need <= 4) launch_row<T, VEC, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+    if (need <= 4) launch_row<T, VEC, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
     else if (need <= 8) launch_row<T, VEC, 8>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
     else if (need <= 16) launch_row<T, VEC, 16>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
     else launch_row<T, VEC, 32>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
@@ -533,11 +880,12 @@ template <typename T>
 alphasparse_status_t launch_spmm_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx,
                                      T beta, T *Y, int ldy, cudaStream_t st, const RowWindow *w) {
     if (ctx->rows == 0 || columns <= 0 || (w && w->count <= 0)) return ALPHA_SPARSE_STATUS_SUCCESS;
-    alphasparse_status_t bs = spmm_split_prepare(ctx, sizeof(T), columns, st);
+    const bool narrow = (size_t)columns * sizeof(T) <= 32 && option(kOptSpmmNarrow);
+    alphasparse_status_t bs = narrow ? spmm_split_prepare(ctx, sizeof(T), columns, st) : spmm_segments_prepare(ctx, sizeof(T), columns, st);
     if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
     bs = col_blocks_ensure(ctx, ctx->spmm, spmm_pick_blocks(ctx, sizeof(T) * (size_t)ctx->cols * (size_t)ldx), st);
     if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
-    if ((size_t)columns * sizeof(T) <= 32 && option(kOptSpmmNarrow)) {
+    if (narrow) {
         launch_narrow<T>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
         ASB_CUDA_OR(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
         return ALPHA_SPARSE_STATUS_SUCCESS;
