@@ -241,8 +241,14 @@ struct SpmmSegments {
     int *d_slot = nullptr;                       // nseg: place of what the segment leaves behind, or -1
     int *d_row = nullptr, *d_first = nullptr;    // rows cut over segments, and the first slot of each (one more closes)
     std::vector<int> seg_row, cross_row, cross_first;  // host copies: what a row window owns
-    void *d_part = nullptr;                      // nslots x columns partial sums
-    size_t part_bytes = 0;
+    // nslots x columns partial sums: one buffer per stream, so that products of one handle on two streams do not meet in
+    // it; a buffer that became too small stays (a recorded graph may hold it) and the next one is at least twice as large.
+    struct Part {
+        cudaStream_t st;
+        void *p;
+        size_t bytes;
+    };
+    std::vector<Part> parts;
 };
 void spmm_segments_destroy(SpmmSegments &s);
 

@@ -160,7 +160,7 @@ struct StreamSegments {
 template <typename T, int VEC, int LPR, bool HAS_BETA>
 __global__ void __launch_bounds__(256, kStreamMinBlocks)
     spmm_stream_kernel(const StreamSegments sg, const int *__restrict__ row_ptr, const int *__restrict__ col,
-                       const T *__restrict__ val, const T *__restrict__ X, int columns, int ldx, T *__restrict__ Y,
+                       const T *__restrict__ val, const T *__restrict__ X, int c0, int columns, int ldx, T *__restrict__ Y,
                        long long ldy, T *__restrict__ part, T alpha, T beta) {
     constexpr int U = kStreamUnroll;
     constexpr int S = 32 / LPR;                        // elements per step
@@ -183,8 +183,8 @@ __global__ void __launch_bounds__(256, kStreamMinBlocks)
         r = (int)first, r_end = (int)min((long long)sg.row1, first + sg.per_warp);
         k = __ldg(row_ptr + r), k_end = __ldg(row_ptr + r_end);
     }
-    const int c = blockIdx.y * (LPR * VEC) + gl * VEC;
-    const bool live = c < columns;
+    const unsigned c = (unsigned)c0 + blockIdx.y * (LPR * VEC) + gl * VEC;
+    const bool live = c < (unsigned)columns;
     const T *Xc = X + (live ? c : 0);  // (lanes beyond the last column read the first and drop it)
 
     // ends of rows r .. r + 31 (lane by lane), and of the 32 rows behind them
@@ -462,7 +462,7 @@ __global__ void spmm_split_kernel(int rows, int blocks, int width, const int *__
 }
 
 void spmm_blocks_destroy(SpmmBlocks &b) {
-    cudaFree(b.d_split);
+    if (b.d_split) cudaFree(b.d_split);  // (even of a null pointer it ends a stream capture)
     b = SpmmBlocks{};
 }
 
@@ -620,7 +620,8 @@ static alphasparse_status_t spmm_split_prepare(DeviceCtx *ctx, size_t tsz, int c
 // ---- segments of a skewed matrix ---------------------------------------------------------------------
 
 void spmm_segments_destroy(SpmmSegments &s) {
-    cudaFree(s.d_seg), cudaFree(s.d_slot), cudaFree(s.d_row), cudaFree(s.d_first), cudaFree(s.d_part);
+    cudaFree(s.d_seg), cudaFree(s.d_slot), cudaFree(s.d_row), cudaFree(s.d_first);
+    for (const SpmmSegments::Part &p : s.parts) cudaFree(p.p);
     s = SpmmSegments{};
 }
 
@@ -694,20 +695,48 @@ static alphasparse_status_t spmm_segments_ensure(DeviceCtx *ctx, cudaStream_t st
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
-// The table (first product of the handle) and room for the partial sums of a product with `columns` columns.
-static alphasparse_status_t spmm_segments_prepare(DeviceCtx *ctx, size_t tsz, int columns, cudaStream_t st) {
-    alphasparse_status_t s = spmm_segments_ensure(ctx, st);
+// The table (made at the first product of the handle) and room for the partial sums of a product with `columns` columns.
+// *part: null when the product has to do with whole rows, because rows are even, because memory for the table is
+// not to be had, or because the stream is being captured and nothing may be allocated now.
+template <typename T>
+static alphasparse_status_t spmm_segments_prepare(DeviceCtx *ctx, int columns, cudaStream_t st, T **part) {
+    *part = nullptr;
     SpmmSegments &sp = ctx->segments;
-    if (s != ALPHA_SPARSE_STATUS_SUCCESS || sp.state != 2) return s;
-    const size_t want = tsz * (size_t)sp.nslots * (size_t)columns;
-    if (sp.part_bytes < want) {
-        cudaFree(sp.d_part);
-        ctx->device_bytes -= (int64_t)sp.part_bytes;
-        sp.d_part = nullptr, sp.part_bytes = 0;
-        ASB_CUDA_OR(device_alloc(&sp.d_part, want), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
-        sp.part_bytes = want;
-        ctx->device_bytes += (int64_t)want;
+    if (sp.state == 1) return ALPHA_SPARSE_STATUS_SUCCESS;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    ASB_CUDA_OR(cudaStreamIsCapturing(st, &capture), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    if (sp.state == 0) {
+        if (capture != cudaStreamCaptureStatusNone) return ALPHA_SPARSE_STATUS_SUCCESS;
+        const alphasparse_status_t s = spmm_segments_ensure(ctx, st);
+        if (s == ALPHA_SPARSE_STATUS_ALLOC_FAILED) return ALPHA_SPARSE_STATUS_SUCCESS;
+        if (s != ALPHA_SPARSE_STATUS_SUCCESS || sp.state != 2) return s;
     }
+    const size_t want = std::max<size_t>(1, sizeof(T) * (size_t)sp.nslots * (size_t)columns);
+    size_t have = 0;
+    for (const SpmmSegments::Part &p : sp.parts) {
+        if (p.st != st) continue;
+        if (p.bytes >= want) {
+            *part = static_cast<T *>(p.p);
+            return ALPHA_SPARSE_STATUS_SUCCESS;
+        }
+        have = std::max(have, p.bytes);
+    }
+    if (capture != cudaStreamCaptureStatusNone) return ALPHA_SPARSE_STATUS_SUCCESS;
+    SpmmSegments::Part grown{st, nullptr, std::max(want, 2 * have)};
+    try {
+        sp.parts.reserve(sp.parts.size() + 1);
+    } catch (...) {
+        return ALPHA_SPARSE_STATUS_SUCCESS;
+    }
+    const cudaError_t e = device_alloc_bytes(&grown.p, grown.bytes);
+    if (e == cudaErrorMemoryAllocation) {
+        (void)cudaGetLastError();
+        return ALPHA_SPARSE_STATUS_SUCCESS;
+    }
+    ASB_CUDA_OR(e, ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    sp.parts.push_back(grown);
+    ctx->device_bytes += (int64_t)grown.bytes;
+    *part = static_cast<T *>(grown.p);
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
@@ -748,10 +777,10 @@ static void launch_row_blocks(DeviceCtx *ctx, T alpha, const T *X, int columns, 
 
 template <typename T, int VEC, int LPR>
 static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
-                       int ldy, cudaStream_t st, const RowWindow *w) {
+                       int ldy, cudaStream_t st, const RowWindow *w, T *part) {
     SpmmSegments &sp = ctx->segments;
     if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
-    if (sp.state != 2 && ctx->spmm.d_split) {
+    if (!part && ctx->spmm.d_split) {
         launch_row_blocks<T, VEC, LPR>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
         if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
         return;
@@ -760,7 +789,7 @@ static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx
     StreamSegments sg{};
     sg.row0 = row0, sg.row1 = row1;
     int64_t groups;
-    if (sp.state == 2) {
+    if (part) {
         // segments that hold anything of the window: the first one that ends at or behind its first row, up to the
         // first one that ends at or behind its end
         const auto b = sp.seg_row.begin() + 1, e = sp.seg_row.end();
@@ -776,16 +805,19 @@ static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx
         groups = (rows + per - 1) / per;
     }
     const T *val = static_cast<const T *>(ctx->d_val);
-    T *part = static_cast<T *>(sp.d_part);
-    const dim3 grid((unsigned)((groups + 7) / 8), (unsigned)((columns + LPR * VEC - 1) / (LPR * VEC)));
-    if (beta == T(0))
-        spmm_stream_kernel<T, VEC, LPR, false><<<grid, 256, 0, st>>>(sg, ctx->d_row_ptr, ctx->d_col, val, X, columns, ldx, Y, ldy,
-                                                                    part, alpha, beta);
-    else
-        spmm_stream_kernel<T, VEC, LPR, true><<<grid, 256, 0, st>>>(sg, ctx->d_row_ptr, ctx->d_col, val, X, columns, ldx, Y, ldy,
-                                                                   part, alpha, beta);
-    count_launch();
-    if (sp.state == 2) {
+    // (one launch for up to 65535 slices of LPR * VEC columns, the most a grid is high)
+    for (int64_t c0 = 0; c0 < columns; c0 += 65535ll * (LPR * VEC)) {
+        const int64_t slices = std::min<int64_t>(65535, (columns - c0 + LPR * VEC - 1) / (LPR * VEC));
+        const dim3 grid((unsigned)((groups + 7) / 8), (unsigned)slices);
+        if (beta == T(0))
+            spmm_stream_kernel<T, VEC, LPR, false><<<grid, 256, 0, st>>>(sg, ctx->d_row_ptr, ctx->d_col, val, X, (int)c0, columns,
+                                                                        ldx, Y, ldy, part, alpha, beta);
+        else
+            spmm_stream_kernel<T, VEC, LPR, true><<<grid, 256, 0, st>>>(sg, ctx->d_row_ptr, ctx->d_col, val, X, (int)c0, columns,
+                                                                       ldx, Y, ldy, part, alpha, beta);
+        count_launch();
+    }
+    if (part) {
         const int64_t l0 = std::lower_bound(sp.cross_row.begin(), sp.cross_row.end(), row0) - sp.cross_row.begin();
         const int64_t l1 = std::lower_bound(sp.cross_row.begin(), sp.cross_row.end(), row1) - sp.cross_row.begin();
         if (l1 > l0) {
@@ -798,13 +830,13 @@ static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx
 
 template <typename T, int VEC>
 static void launch_row_lanes(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
-                             int ldy, cudaStream_t st, const RowWindow *w) {
+                             int ldy, cudaStream_t st, const RowWindow *w, T *part) {
     // smallest group (4 .. 32 lanes) whose lanes cover the dense columns in one pass, if any
     const int need = (columns + VEC - 1) / VEC;
-    if (need <= 4) launch_row<T, VEC, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
-    else if (need <= 8) launch_row<T, VEC, 8>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
-    else if (need <= 16) launch_row<T, VEC, 16>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
-    else launch_row<T, VEC, 32>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+    if (need <= 4) launch_row<T, VEC, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+    else if (need <= 8) launch_row<T, VEC, 8>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+    else if (need <= 16) launch_row<T, VEC, 16>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+    else launch_row<T, VEC, 32>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
 }
 
 template <typename T, int LANES, int KC, bool ALIGNED>
@@ -881,7 +913,8 @@ alphasparse_status_t launch_spmm_row(DeviceCtx *ctx, T alpha, const T *X, int co
                                      T beta, T *Y, int ldy, cudaStream_t st, const RowWindow *w) {
     if (ctx->rows == 0 || columns <= 0 || (w && w->count <= 0)) return ALPHA_SPARSE_STATUS_SUCCESS;
     const bool narrow = (size_t)columns * sizeof(T) <= 32 && option(kOptSpmmNarrow);
-    alphasparse_status_t bs = narrow ? spmm_split_prepare(ctx, sizeof(T), columns, st) : spmm_segments_prepare(ctx, sizeof(T), columns, st);
+    T *part = nullptr;
+    alphasparse_status_t bs = narrow ? spmm_split_prepare(ctx, sizeof(T), columns, st) : spmm_segments_prepare<T>(ctx, columns, st, &part);
     if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
     bs = col_blocks_ensure(ctx, ctx->spmm, spmm_pick_blocks(ctx, sizeof(T) * (size_t)ctx->cols * (size_t)ldx), st);
     if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
@@ -897,12 +930,12 @@ alphasparse_status_t launch_spmm_row(DeviceCtx *ctx, T alpha, const T *X, int co
     };
     // Widest 16-byte pack the shapes and alignments allow.
     if constexpr (sizeof(T) == 4) {
-        if (fits(4)) launch_row_lanes<T, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
-        else if (fits(2)) launch_row_lanes<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
-        else launch_row_lanes<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+        if (fits(4)) launch_row_lanes<T, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+        else if (fits(2)) launch_row_lanes<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+        else launch_row_lanes<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
     } else {
-        if (fits(2)) launch_row_lanes<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
-        else launch_row_lanes<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+        if (fits(2)) launch_row_lanes<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+        else launch_row_lanes<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
     }
     ASB_CUDA_OR(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     return ALPHA_SPARSE_STATUS_SUCCESS;

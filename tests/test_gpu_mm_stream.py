@@ -1,0 +1,135 @@
+"""The row-major dense-block product's element-stream kernel: edges of its batches and segments, rows cut over segments,
+more column slices than one grid holds, and the calls that may not allocate."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from alsparse_b200 import capi, spblas, synth
+from gpu_util import TORCH, make_handle
+from helpers import assert_rows_close, mm_scale
+
+pytestmark = pytest.mark.gpu
+
+
+def lengths(shape):
+    if shape == "even":  # whole rows per warp, empty ones among them
+        lens = synth.rowlen_poisson(21, 9001, 6.0, 900).copy()
+        lens[::13] = 0
+        return lens
+    # rows around the lengths at which a row may be cut, long rows side by side, runs of empty rows at both ends
+    rng = np.random.default_rng(3)
+    lens = rng.choice([0, 0, 1, 2, 7, 31, 32, 33, 63, 64, 65, 66, 127], 4000).astype(np.int32)
+    lens[:40] = 0
+    lens[-50:] = 0
+    lens[[40, 41, 1000, 1001, 3949]] = [900, 257, 2000, 256, 1999]
+    return lens
+
+
+def multiply(kind, A, alpha, X, columns, ldx, beta, Y, ldy):
+    assert spblas.mm(kind, 0, alpha, A, spblas.descr(), capi.ROW_MAJOR, X, columns, ldx, beta, Y, ldy) == capi.SUCCESS, \
+        spblas.last_error()
+
+
+def check(kind, m, A, columns, pad=0, alpha=1.5, beta=0.5, call=multiply):
+    ldx, ldy = columns + pad, columns + pad
+    X, Y0 = synth.vector(kind, 5, 3, m.cols * ldx), synth.vector(kind, 5, 4, m.nrows * ldy)
+    # (long fp32 rows: the oracle in double precision spends no tolerance on its own rounding)
+    f = np.float64
+    ref = oracle.gemm("d", "row", m.rows_start, m.rows_end, m.col, m.val.astype(f), alpha, X.astype(f), columns, ldx, beta,
+                      Y0.astype(f), ldy)
+    dX, dY = torch.from_numpy(X).cuda(), torch.from_numpy(Y0).cuda()
+    call(kind, A, alpha, dX, columns, ldx, beta, dY, ldy)
+    torch.cuda.synchronize()
+    scale = mm_scale(m.ptr, m.col, m.val, X, columns, ldx, alpha, beta, Y0, ldy)
+    shape = (m.nrows, ldy)
+    assert_rows_close(kind, dY.cpu().numpy().reshape(shape)[:, :columns].reshape(-1),
+                      ref.reshape(shape)[:, :columns].reshape(-1), scale.reshape(-1), f"{columns} columns")
+
+
+@pytest.mark.parametrize("kind", ["s", "d"])
+@pytest.mark.parametrize("shape", ["even", "skewed"])
+def test_batches_segments_and_cut_rows(kind, shape):
+    m = synth.from_lengths(kind, 21, lengths(shape), 2500)
+    A = make_handle(kind, m)
+    for columns, pad in ((9, 0), (12, 0), (16, 0), (20, 3), (33, 0), (64, 0), (130, 2)):
+        check(kind, m, A, columns, pad)
+    check(kind, m, A, 24, beta=0.0)
+    spblas.destroy(A)
+
+
+def test_more_column_slices_than_a_grid_is_high():
+    columns = 65535 * 32 + 1  # odd: single elements, 32 lanes wide
+    lens = np.array([2, 0, 3], np.int32)
+    m = synth.from_lengths("s", 4, lens, 3)
+    A = make_handle("s", m)
+    X = torch.rand(3, columns, device="cuda")
+    Y = torch.zeros(3, columns, device="cuda")
+    multiply("s", A, 1.0, X, columns, columns, 0.0, Y, columns)
+    dense = np.zeros((3, 3))
+    np.add.at(dense, (np.repeat(np.arange(3), lens), m.col), m.val)
+    ref = torch.from_numpy(dense).cuda() @ X.double()
+    assert float((Y - ref).abs().max()) <= 1e-5 * 3
+    spblas.destroy(A)
+
+
+@pytest.mark.parametrize("kind", ["s", "d"])
+def test_products_that_may_not_allocate(kind):
+    """A capture before and after the segment table exists, a wider product behind a recorded one, a refused allocation."""
+    m = synth.from_lengths(kind, 21, lengths("skewed"), 2500)
+    lib = capi.load()
+    side = torch.cuda.Stream()
+
+    def captured(*args):
+        side.wait_stream(torch.cuda.current_stream())
+        graph = torch.cuda.CUDAGraph()
+        spblas.set_stream(side.cuda_stream)
+        try:
+            with torch.cuda.stream(side), torch.cuda.graph(graph, stream=side):
+                multiply(*args)
+            graph.replay()
+        finally:
+            spblas.set_stream(None)
+        torch.cuda.synchronize()
+
+    def denied(*args):
+        lib.alphasparse_cuda_debug_fail_alloc(1)
+        try:
+            multiply(*args)
+        finally:
+            lib.alphasparse_cuda_debug_fail_alloc(0)
+
+    even = synth.from_lengths(kind, 21, lengths("even"), 2500)
+    A = make_handle(kind, even)
+    for columns in (24, 40):
+        check(kind, even, A, columns)  # (loads the kernels)
+    spblas.destroy(A)
+    A = make_handle(kind, m)
+    check(kind, m, A, 24, call=captured)
+    check(kind, m, A, 24, call=denied)
+    spblas.set_stream(side.cuda_stream)
+    try:
+        check(kind, m, A, 24)  # the table, and room for 24 columns on this stream
+    finally:
+        spblas.set_stream(None)
+    check(kind, m, A, 24, call=captured)
+    check(kind, m, A, 40, call=captured)  # no room for 40
+
+    # a recorded product stays usable behind a wider one
+    x, y, z = (torch.rand(n, dtype=TORCH[kind], device="cuda") for n in (m.cols * 24, m.nrows * 24, m.cols * 128))
+    want = torch.zeros_like(y)
+    graph = torch.cuda.CUDAGraph()
+    side.wait_stream(torch.cuda.current_stream())
+    spblas.set_stream(side.cuda_stream)
+    try:
+        with torch.cuda.stream(side):
+            multiply(kind, A, 1.0, x, 24, 24, 0.0, want, 24)
+            with torch.cuda.graph(graph, stream=side):
+                multiply(kind, A, 1.0, x, 24, 24, 0.0, y, 24)
+            multiply(kind, A, 1.0, z, 128, 128, 0.0, torch.zeros(m.nrows * 128, dtype=TORCH[kind], device="cuda"), 128)
+            graph.replay()
+            side.synchronize()
+    finally:
+        spblas.set_stream(None)
+    assert torch.equal(y, want)
+    spblas.destroy(A)
