@@ -136,6 +136,66 @@ constexpr int kMergeItemsD = 7;  // double
 // ask for (four blocks per SM must still fit in the 227 KB an SM offers).
 constexpr int kRowTile = 128;
 constexpr size_t kRowTileMaxSmem = 56 * 1024;
+constexpr int kRowTileSmall = 32;               // rows per block where tiles are large (launch_rowtile)
+constexpr size_t kSmemPerSm = 228 * 1024;
+
+struct DeviceCtx;
+int rowtile_cap(const DeviceCtx *ctx, int tile);
+size_t rowtile_smem_bytes(const DeviceCtx *ctx, int tile);
+
+// Bulk copy global -> shared counted on an mbarrier (shared addresses as 32-bit numbers; both addresses and the size
+// are multiples of 16 bytes), and one poll of the mbarrier.
+__device__ __forceinline__ unsigned smem_u32(const void *p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void bulk_copy_g2s(unsigned dst, const void *src, unsigned bytes, unsigned bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                 :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
+    unsigned ok;
+    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+
+// A block of TILE threads brings the offsets, columns and values of rows [r0, r0 + nr) into shared memory and waits for
+// them, with a limit.  The element range is widened to multiples of four elements so that source addresses and sizes
+// are multiples of 16 bytes, as the bulk copy requires; the arrays carry a zero tail for that.  False: the thread must
+// leave without touching the tile (the error word says why).
+template <typename T, int TILE>
+__device__ __forceinline__ bool stage_row_tile(int r0, int nr, const int *__restrict__ row_ptr, const int *__restrict__ col,
+                                               const T *__restrict__ val, T *s_val, int *s_col, int *s_ptr, int cap,
+                                               int *__restrict__ status) {
+    __shared__ __align__(8) unsigned long long s_bar;
+    __shared__ int s_oversize;
+    const unsigned bar = smem_u32(&s_bar);
+    if (threadIdx.x == 0) {
+        const int start = __ldg(row_ptr + r0), end = __ldg(row_ptr + r0 + nr);
+        const int a0 = start & ~3;
+        int n = ((end + 3) & ~3) - a0;
+        s_oversize = n > cap;
+        if (n > cap) {  // cannot happen for a handle analysed by this library; refuse rather than overrun
+            atomicExch(status, 1);
+            n = 0;
+        }
+        const unsigned ptr_bytes = (unsigned)(((nr + 1 + 3) & ~3) * sizeof(int));
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        const unsigned bytes = ptr_bytes + (unsigned)n * (unsigned)(sizeof(int) + sizeof(T));
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
+        bulk_copy_g2s(smem_u32(s_ptr), row_ptr + r0, ptr_bytes, bar);
+        if (n > 0) {
+            bulk_copy_g2s(smem_u32(s_col), col + a0, (unsigned)n * sizeof(int), bar);
+            bulk_copy_g2s(smem_u32(s_val), val + a0, (unsigned)n * sizeof(T), bar);
+        }
+    }
+    __syncthreads();
+    bool arrived = false;
+    for (int spin = 0; spin < (1 << 22) && !arrived; spin++) arrived = mbar_try_wait(bar, 0);
+    if (!arrived && threadIdx.x == 0) atomicExch(status, 2);
+    return arrived && !s_oversize;  // (oversize: nothing was staged, the whole block leaves)
+}
 
 // Where a kernel delivers finished y rows besides its own y: the next-x buffer of every GPU of the
 // row partition (peer-mapped device pointers), row r of this block landing at element row_off + r.
@@ -269,6 +329,7 @@ struct DeviceCtx {
     double mean_row_quads = 0.0;  // aligned 4-element groups a row touches, on average
     double shifted_rows = 0.0;    // share of sampled elements whose next-row twin sits one column to the right
     int64_t max_tile_span = 0;    // largest quad-aligned element span of kRowTile consecutive rows
+    int64_t max_small_span = 0;   // ... of kRowTileSmall
     int algorithm = ALPHA_SPARSE_CUDA_ALG_VECTOR;
     int lanes = 4;
 

@@ -143,84 +143,35 @@ __global__ void __launch_bounds__(256, VectorShape<LANES>::MIN_BLOCKS)
 
 // ---- row-tile kernel ----------------------------------------------------------------------------
 //
-// One block stages the column indices, values and offsets of kRowTile consecutive rows in
-// shared memory with three bulk asynchronous copies (cp.async.bulk global -> shared, completion
-// counted in bytes on an mbarrier), then every thread walks ONE row out of shared memory.
-// Compared with the vector kernel this turns the x gathers of a banded matrix into coalesced
-// accesses (neighbouring lanes = neighbouring rows = neighbouring columns), which is what the
-// 27-point stencil needs: there the vector kernel is limited by L1 wavefronts, not by HBM.
-// Several blocks are resident per SM, so the copies of one overlap the arithmetic of another.
+// One block stages the column indices, values and offsets of TILE consecutive rows in shared memory with three bulk
+// asynchronous copies (cp.async.bulk global -> shared, completion counted in bytes on an mbarrier; stage_row_tile), then
+// every thread walks ONE row out of shared memory.  Compared with the vector kernel this turns the x gathers of a banded
+// matrix into coalesced accesses (neighbouring lanes = neighbouring rows = neighbouring columns), which is what the
+// 27-point stencil needs: there the vector kernel is limited by L1 wavefronts, not by HBM.  Several blocks are resident
+// per SM, so the copies of one overlap the arithmetic of another.
 //
-// The element range of a tile is widened to multiples of four elements so that source
-// addresses and sizes are multiples of 16 bytes, as the bulk copy requires; the arrays carry a
-// zero tail for that.  The wait on the mbarrier is bounded: if it runs out the block records
-// an error word and leaves without touching y.
-
-__device__ __forceinline__ unsigned smem_u32(const void *p) {
-    return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void bulk_copy_g2s(unsigned dst, const void *src, unsigned bytes, unsigned bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 :: "r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
-    unsigned ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-
-template <typename T, bool HAS_BETA, bool PUSH>
-__global__ void __launch_bounds__(kRowTile)
+// TILE is 32 (a block is one warp, and none waits for another's rows or copies) where that many rows are enough for the
+// 32 blocks an SM holds to fill its shared memory, else 128 (fewer copies, and all the warps an SM can have).
+// Measured (B200, us, tiles of 128 -> tiles of 32): 27-point stencil fp64 160^3 237 -> 223 (6.24 TB/s), 61^3 24.4 -> 20.5, fp32
+// 100^3 47.2 -> 43.9; banded fp64 of 2e6 rows x 25 / 21 / 17 elements 134 / 112 / 89 -> 123 / 104 / 87.  Shorter rows lose:
+// 4e6 rows x 3 elements 71 -> 82, 400,000 rows x 4 in fp32 10.9 -> 12.8.  Several warps with a tile each in one block were
+// slower than either (160^3: 250 us).
+template <typename T, int TILE, bool HAS_BETA, bool PUSH>
+__global__ void __launch_bounds__(TILE)
     spmv_rowtile_kernel(int rows, const int *__restrict__ row_ptr, const int *__restrict__ col,
                         const T *__restrict__ val, const T *__restrict__ x, T *__restrict__ y, T alpha,
                         T beta, int cap, int *__restrict__ status, PeerPush push) {
     extern __shared__ __align__(128) unsigned char smem[];
     T *s_val = reinterpret_cast<T *>(smem);
-    int *s_col = reinterpret_cast<int *>(smem + (size_t)cap * sizeof(T));
+    int *s_col = reinterpret_cast<int *>(s_val + cap);
     int *s_ptr = s_col + cap;
-    unsigned long long *s_bar = reinterpret_cast<unsigned long long *>(s_ptr + kRowTile + 4);
-    __shared__ int s_oversize;
 
     const int tid = threadIdx.x;
-    const int r0 = blockIdx.x * kRowTile;
-    const int nr = min(kRowTile, rows - r0);
-    const unsigned bar = smem_u32(s_bar);
-
-    if (tid == 0) {
-        const int start = __ldg(row_ptr + r0), end = __ldg(row_ptr + r0 + nr);
-        const int a0 = start & ~3;
-        int n = ((end + 3) & ~3) - a0;
-        s_oversize = n > cap;
-        if (n > cap) {  // cannot happen for a handle analysed by this library; refuse rather than overrun
-            atomicExch(status, 1);
-            n = 0;
-        }
-        const unsigned ptr_bytes = (unsigned)(((nr + 1 + 3) & ~3) * sizeof(int));
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        const unsigned bytes = ptr_bytes + (unsigned)n * (unsigned)(sizeof(int) + sizeof(T));
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" :: "r"(bar), "r"(bytes) : "memory");
-        bulk_copy_g2s(smem_u32(s_ptr), row_ptr + r0, ptr_bytes, bar);
-        if (n > 0) {
-            bulk_copy_g2s(smem_u32(s_col), col + a0, (unsigned)n * sizeof(int), bar);
-            bulk_copy_g2s(smem_u32(s_val), val + a0, (unsigned)n * sizeof(T), bar);
-        }
-    }
-    __syncthreads();
-
-    bool arrived = false;
-    for (int spin = 0; spin < (1 << 22); spin++) {
-        if (mbar_try_wait(bar, 0)) {
-            arrived = true;
-            break;
-        }
-    }
-    if (!arrived) {
-        if (tid == 0) atomicExch(status, 2);
-        return;
-    }
-    if (s_oversize) return;  // nothing was staged: the whole block leaves before it touches the tile or x
+    const int r0 = blockIdx.x * TILE;
+    const int nr = min(TILE, rows - r0);
+    T old = T(0);  // requested before the wait: its latency hides behind the copies
+    if (HAS_BETA && tid < nr) old = __ldcs(y + r0 + tid);
+    if (!stage_row_tile<T, TILE>(r0, nr, row_ptr, col, val, s_val, s_col, s_ptr, cap, status)) return;
 
     const int a0 = s_ptr[0] & ~3;
     const int b = tid < nr ? s_ptr[tid] - a0 : 0, e = tid < nr ? s_ptr[tid + 1] - a0 : 0;
@@ -266,7 +217,7 @@ __global__ void __launch_bounds__(kRowTile)
         }
         const int r = r0 + tid;
         T out = alpha * ((acc0 + acc1) + (acc2 + acc3));
-        if (HAS_BETA) out = fma(beta, y[r], out);
+        if (HAS_BETA) out = fma(beta, old, out);
         __stcs(y + r, out);
         if (PUSH) {  // neighbouring lanes hold neighbouring rows: coalesced stores into every peer's next x
 #pragma unroll 1
@@ -594,10 +545,10 @@ __global__ void scale_kernel(long long n, T *__restrict__ y, T beta) {
 
 // out[0] = max row length, out[1] = empty rows, out[2] = aligned quads touched (summed over
 // rows), out[3] = rows whose end offset is below their start offset (malformed input),
-// out[5] = largest quad-aligned element span of a tile of kRowTile consecutive rows.
+// out[5], out[8] = largest quad-aligned element span of a tile of kRowTile / kRowTileSmall consecutive rows.
 __global__ void row_stats_kernel(int rows, const int *__restrict__ row_ptr,
                                  unsigned long long *__restrict__ out) {
-    unsigned long long mx = 0, empty = 0, quads = 0, bad = 0, span = 0;
+    unsigned long long mx = 0, empty = 0, quads = 0, bad = 0, span = 0, span_small = 0;
     for (long long r = (long long)blockIdx.x * blockDim.x + threadIdx.x; r < rows;
          r += (long long)gridDim.x * blockDim.x) {
         const int s = row_ptr[r], e = row_ptr[r + 1];
@@ -609,20 +560,23 @@ __global__ void row_stats_kernel(int rows, const int *__restrict__ row_ptr,
         mx = len > mx ? len : mx;
         if (len == 0) empty++;
         else quads += (unsigned long long)(((e + 3) >> 2) - (s >> 2));
-        if (r % kRowTile == 0) {
-            const long long last = r + kRowTile < rows ? r + kRowTile : rows;
-            const int te = row_ptr[last];
-            if (te >= s) {
-                const unsigned long long sp = (unsigned long long)(((te + 3) & ~3) - (s & ~3));
-                span = sp > span ? sp : span;
-            }
-        }
+        auto widest = [&](int tile, unsigned long long &most) {
+            if (r % tile != 0) return;
+            const int te = row_ptr[r + tile < rows ? r + tile : rows];
+            if (te < s) return;
+            const unsigned long long sp = (unsigned long long)(((te + 3) & ~3) - (s & ~3));
+            most = sp > most ? sp : most;
+        };
+        widest(kRowTile, span);
+        widest(kRowTileSmall, span_small);
     }
     for (int o = 16; o > 0; o >>= 1) {
         const unsigned long long m2 = __shfl_xor_sync(0xffffffffu, mx, o);
         mx = m2 > mx ? m2 : mx;
         const unsigned long long s2 = __shfl_xor_sync(0xffffffffu, span, o);
         span = s2 > span ? s2 : span;
+        const unsigned long long s3 = __shfl_xor_sync(0xffffffffu, span_small, o);
+        span_small = s3 > span_small ? s3 : span_small;
         empty += __shfl_xor_sync(0xffffffffu, empty, o);
         quads += __shfl_xor_sync(0xffffffffu, quads, o);
         bad += __shfl_xor_sync(0xffffffffu, bad, o);
@@ -630,6 +584,7 @@ __global__ void row_stats_kernel(int rows, const int *__restrict__ row_ptr,
     if ((threadIdx.x & 31) == 0) {
         atomicMax(out + 0, mx);
         atomicMax(out + 5, span);
+        atomicMax(out + 8, span_small);
         if (empty) atomicAdd(out + 1, empty);
         if (quads) atomicAdd(out + 2, quads);
         if (bad) atomicAdd(out + 3, bad);
@@ -717,11 +672,13 @@ __global__ void tile_key_kernel(long long tiles, const MergeCoord *__restrict__ 
 
 // ---- analysis (host) ------------------------------------------------------------------------------
 
-// Dynamic shared memory of one row-tile block: values | columns | offsets (+4 pad) | mbarrier.
-static size_t rowtile_smem_bytes(const DeviceCtx *ctx) {
-    const size_t cap = (size_t)((ctx->max_tile_span + 3) & ~3ll);
+// Elements one tile of `tile` rows makes room for, and the block's dynamic shared memory: values | columns | offsets.
+int rowtile_cap(const DeviceCtx *ctx, int tile) {
+    return (int)(((tile == kRowTile ? ctx->max_tile_span : ctx->max_small_span) + 3) & ~3ll);
+}
+size_t rowtile_smem_bytes(const DeviceCtx *ctx, int tile) {
     const size_t tsz = ctx->datatype == ALPHA_SPARSE_DATATYPE_DOUBLE ? 8 : 4;
-    return cap * (tsz + sizeof(int)) + (kRowTile + 4) * sizeof(int) + 16;
+    return (size_t)rowtile_cap(ctx, tile) * (tsz + sizeof(int)) + (tile + 4) * sizeof(int);
 }
 
 static int pick_lanes(double mean_quads) {
@@ -919,7 +876,7 @@ alphasparse_status_t ctx_analyse(DeviceCtx *ctx) {
     ctx->max_row_nnz = 0, ctx->empty_rows = ctx->rows, ctx->mean_row_nnz = 0.0;
     if (ctx->rows == 0) return ALPHA_SPARSE_STATUS_SUCCESS;
 
-    unsigned long long *d_out = ctx->d_stats, h_out[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+    unsigned long long *d_out = ctx->d_stats, h_out[9] = {};
     if (!d_out) ASB_CUDA_OR(device_alloc(&d_out, sizeof(h_out)), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
     cudaError_t e = cudaMemsetAsync(d_out, 0, sizeof(h_out), st);
     if (e == cudaSuccess) {
@@ -954,14 +911,14 @@ alphasparse_status_t ctx_analyse(DeviceCtx *ctx) {
     ctx->empty_rows = (int64_t)h_out[1];
     ctx->mean_row_nnz = (double)ctx->nnz / (double)ctx->rows;
     ctx->mean_row_quads = (double)h_out[2] / (double)ctx->rows;
-    ctx->max_tile_span = (int64_t)h_out[5];
+    ctx->max_tile_span = (int64_t)h_out[5], ctx->max_small_span = (int64_t)h_out[8];
     ctx->shifted_rows = h_out[7] ? (double)h_out[6] / (double)h_out[7] : 0.0;
     ctx->lanes = pick_lanes(ctx->mean_row_quads);
 
     // A row longer than eight passes of its lane group would leave that group running long
     // after the rest of the grid has drained: switch to equal-work tiles.
     int alg = forced_algorithm();
-    const bool rowtile_fits = rowtile_smem_bytes(ctx) <= kRowTileMaxSmem;
+    const bool rowtile_fits = rowtile_smem_bytes(ctx, kRowTile) <= kRowTileMaxSmem;
     if (alg == ALPHA_SPARSE_CUDA_ALG_ROWTILE && !rowtile_fits) alg = ALPHA_SPARSE_CUDA_ALG_AUTO;
     if (alg == ALPHA_SPARSE_CUDA_ALG_AUTO) {
         const int64_t comfortable = (int64_t)ctx->lanes * 4 * 8;
@@ -1127,19 +1084,19 @@ static void launch_merge(DeviceCtx *ctx, T alpha, const T *x, T beta, T *y, cuda
     }
 }
 
-template <typename T>
-static alphasparse_status_t launch_rowtile(DeviceCtx *ctx, T alpha, const T *x, T beta, T *y,
-                                           cudaStream_t st, const PeerPush *pushp, const RowWindow &w) {
-    const int cap = (int)((ctx->max_tile_span + 3) & ~3ll);
-    const size_t smem = rowtile_smem_bytes(ctx);
+template <typename T, int TILE>
+static alphasparse_status_t launch_rowtile_as(DeviceCtx *ctx, T alpha, const T *x, T beta, T *y, cudaStream_t st,
+                                              const PeerPush *pushp, const RowWindow &w) {
+    const int cap = rowtile_cap(ctx, TILE);
+    const size_t smem = rowtile_smem_bytes(ctx, TILE);
     const T *val = static_cast<const T *>(ctx->d_val);
-    const unsigned blocks = (unsigned)((w.count + kRowTile - 1) / kRowTile);
+    const unsigned blocks = (unsigned)((w.count + TILE - 1) / TILE);
     const bool in_kernel = pushp && !pushp->after;
     const PeerPush push = in_kernel ? *pushp : PeerPush{};
     const int which = (beta == T(0) ? 0 : 1) + (in_kernel ? 2 : 0);
-    decltype(&spmv_rowtile_kernel<T, false, false>) variants[4] = {
-        spmv_rowtile_kernel<T, false, false>, spmv_rowtile_kernel<T, true, false>,
-        spmv_rowtile_kernel<T, false, true>, spmv_rowtile_kernel<T, true, true>};
+    decltype(&spmv_rowtile_kernel<T, TILE, false, false>) variants[4] = {
+        spmv_rowtile_kernel<T, TILE, false, false>, spmv_rowtile_kernel<T, TILE, true, false>,
+        spmv_rowtile_kernel<T, TILE, false, true>, spmv_rowtile_kernel<T, TILE, true, true>};
     auto kernel = variants[which];
     // The opt-in limit is a property of the kernel, shared by all handles: only ever raise it.
     static std::atomic<size_t> granted[4] = {{0}, {0}, {0}, {0}};
@@ -1152,11 +1109,20 @@ static alphasparse_status_t launch_rowtile(DeviceCtx *ctx, T alpha, const T *x, 
     if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
     // w.begin is a multiple of kRowTile (the caller's duty): tiles, and the 16-byte alignment of the
     // offset copies, are the same as in a full launch
-    kernel<<<blocks, kRowTile, smem, st>>>((int)w.count, ctx->d_row_ptr + w.begin, ctx->d_col, val, x,
-                                           y + w.begin, alpha, beta, cap, ctx->d_status, push);
+    kernel<<<blocks, TILE, smem, st>>>((int)w.count, ctx->d_row_ptr + w.begin, ctx->d_col, val, x, y + w.begin, alpha, beta, cap,
+                                       ctx->d_status, push);
     if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
     count_launch();
     return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
+template <typename T>
+static alphasparse_status_t launch_rowtile(DeviceCtx *ctx, T alpha, const T *x, T beta, T *y, cudaStream_t st,
+                                           const PeerPush *push, const RowWindow &w) {
+    const size_t small = rowtile_smem_bytes(ctx, kRowTileSmall);  // (a block takes 1 KB for itself)
+    if (small <= kRowTileMaxSmem && small + 1024 >= kSmemPerSm / 32)
+        return launch_rowtile_as<T, kRowTileSmall>(ctx, alpha, x, beta, y, st, push, w);
+    return launch_rowtile_as<T, kRowTile>(ctx, alpha, x, beta, y, st, push, w);
 }
 
 template <typename T>
