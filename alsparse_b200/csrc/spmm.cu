@@ -1035,6 +1035,86 @@ static void launch_col(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx
     if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
 }
 
+// ---- column-major operands, banded matrix ---------------------------------------------------------------
+//
+// When neighbouring rows hold neighbouring columns (stencils, banded matrices in natural order) a lane per row gathers
+// coalesced from every column of X as it is stored, so nothing needs transposing: a warp stages the offsets, columns and
+// values of kRowTileSmall rows in shared memory once (as the row-tile SpMV does, spmv.cu) and walks them for KC dense columns
+// at a time.  A is read once from HBM, X and Y once each; what bounds it is the latency of the gathers (they come out of
+// L2: shared memory leaves L1 little room), so U elements of a row are taken together, U * KC gathers in flight.
+// Measured (B200, 27-point stencil 80^3, us, through transposes -> here): fp64 1 / 2 / 4 / 6 / 13 / 32 columns 87 / 115 / 159 /
+// 211 / 316 / 569 -> 40 / 42 / 52 / 60 / 118 / 220; fp32 3 / 6 / 32 columns 117 / 173 / 264 -> 33 / 50 / 181; 20^3 fp32 x 32
+// columns 25 -> 9.  U = 2 for eight columns took 310 us for 32 (3: 220, 4: 218 in fp64, but 181 -> 218 in fp32); U = 2 / 4
+// for six 81 / 73 (6: 60).  Blocks of four warps made no difference, fewer resident warps (more L1) lost 20-80 %.
+template <typename T, int KC, bool HAS_BETA>
+__global__ void __launch_bounds__(kRowTileSmall)
+    spmm_col_tile_kernel(int rows, const int *__restrict__ row_ptr, const int *__restrict__ col, const T *__restrict__ val,
+                         const T *__restrict__ X, int columns, long long ldx, T *__restrict__ Y, long long ldy, T alpha,
+                         T beta, int cap, int *__restrict__ status) {
+    constexpr int U = KC >= 8 ? 3 : KC >= 4 ? 6 : 8;
+    extern __shared__ __align__(128) unsigned char smem[];
+    T *s_val = reinterpret_cast<T *>(smem);
+    int *s_col = reinterpret_cast<int *>(s_val + cap);
+    int *s_ptr = s_col + cap;
+
+    const int tid = threadIdx.x;
+    const int r0 = blockIdx.x * kRowTileSmall;
+    const int nr = min(kRowTileSmall, rows - r0);
+    if (!stage_row_tile<T, kRowTileSmall>(r0, nr, row_ptr, col, val, s_val, s_col, s_ptr, cap, status) || tid >= nr) return;
+
+    const int a0 = s_ptr[0] & ~3;
+    const int b = s_ptr[tid] - a0, e = s_ptr[tid + 1] - a0;
+    const long long r = r0 + tid;
+    for (long long c0 = (long long)blockIdx.y * KC; c0 < columns; c0 += (long long)gridDim.y * KC) {
+        const int live = (int)min((long long)KC, columns - c0);
+        const T *x[KC];  // (beyond the last column: the last one again, dropped below)
+        T acc[KC], old[KC];
+#pragma unroll
+        for (int i = 0; i < KC; i++) {
+            x[i] = X + (c0 + min(i, live - 1)) * ldx;
+            acc[i] = T(0), old[i] = T(0);
+            if (HAS_BETA && i < live) old[i] = __ldcs(Y + (c0 + i) * ldy + r);
+        }
+        for (int k = b; k < e; k += U) {
+            T v[U], xv[U][KC];
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (k + u < e) {
+                    const int c = s_col[k + u];
+                    v[u] = s_val[k + u];
+#pragma unroll
+                    for (int i = 0; i < KC; i++) xv[u][i] = __ldg(x[i] + c);
+                }
+#pragma unroll
+            for (int u = 0; u < U; u++)
+                if (k + u < e) {
+#pragma unroll
+                    for (int i = 0; i < KC; i++) acc[i] = fma(v[u], xv[u][i], acc[i]);
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < KC; i++)
+            if (i < live) __stcs(Y + (c0 + i) * ldy + r, HAS_BETA ? fma(beta, old[i], alpha * acc[i]) : alpha * acc[i]);
+    }
+}
+
+template <typename T, int KC>
+static alphasparse_status_t launch_col_tile(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y, int ldy,
+                                            cudaStream_t st) {
+    auto kernel = beta == T(0) ? spmm_col_tile_kernel<T, KC, false> : spmm_col_tile_kernel<T, KC, true>;
+    // A warp does all columns of its rows; where the rows alone do not fill the chip they are shared out.
+    const int64_t tiles = (ctx->rows + kRowTileSmall - 1) / kRowTileSmall, chunks = (columns + KC - 1) / KC;
+    const int64_t share = std::min(chunks, std::max<int64_t>(1, 148 * 32 / tiles));
+    if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
+    kernel<<<dim3((unsigned)tiles, (unsigned)share), kRowTileSmall, rowtile_smem_bytes(ctx, kRowTileSmall), st>>>(
+        (int)ctx->rows, ctx->d_row_ptr, ctx->d_col, static_cast<const T *>(ctx->d_val), X, columns, ldx, Y, ldy, alpha, beta,
+        rowtile_cap(ctx, kRowTileSmall), ctx->d_status);
+    if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
+    count_launch();
+    ASB_CUDA_OR(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
 // B[f * ld_b + s] = A[s * ld_a + f] for f < n_fast, s < n_slow: a column-major operand (f = row, s = dense column)
 // into a row-major one, or back (f = dense column, s = row).  32 x 32 tiles through shared memory; the tiles along the
 // longer of the two extents are numbered by blockIdx.x (`slow_on_x`), whose range is the wide one.
@@ -1084,6 +1164,16 @@ template <typename T>
 alphasparse_status_t launch_spmm_col(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
                                      int ldy, cudaStream_t st) {
     if (ctx->rows == 0 || columns <= 0) return ALPHA_SPARSE_STATUS_SUCCESS;
+    if (ctx->algorithm == ALPHA_SPARSE_CUDA_ALG_ROWTILE && ctx->shifted_rows >= 0.5 && ctx->nnz > 0 &&
+        rowtile_smem_bytes(ctx, kRowTileSmall) <= 48 * 1024) {
+        const int passes = (columns + 7) / 8, per = (columns + passes - 1) / passes;  // columns in equal groups of at most 8
+        if (per <= 1) return launch_col_tile<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st);
+        if (per <= 2) return launch_col_tile<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st);
+        if (per <= 3) return launch_col_tile<T, 3>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st);
+        if (per <= 4) return launch_col_tile<T, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st);
+        if (per <= 6) return launch_col_tile<T, 6>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st);
+        return launch_col_tile<T, 8>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st);
+    }
     // The kernel below gathers one x element per (stored element, dense column): four L2 requests per element and
     // pass of four columns, where the row-major kernels take a whole X row with one or two (2^21 rows of 32 elements
     // times 8 / 64 fp32 columns: 2.0 / 16.2 ms column-major against 0.6 / 3.5 ms row-major).  From spmm_col_via_row
