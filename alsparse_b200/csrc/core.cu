@@ -833,6 +833,8 @@ static alphasparse_status_t csr_shadow_of(const alphasparse_matrix_t A, alphaspa
 // overlap.  Three streams: x and the y0 pieces go in on one, the windows run on the library stream as their inputs
 // land, every finished piece of y leaves on the third while the next window is being multiplied (PCIe is full
 // duplex).  The call still returns only when all of y is back in host memory.
+// Pageable vectors go through the page-locked rings (transfer.cu): fp64 400,000 / 3e6 rows of 8 elements with beta != 0
+// 0.84 / 6.2 -> 0.35 / 3.7 ms.
 // The number of windows follows the size of y: pieces of at least pipe_min_piece_kb, at most pipe_max_windows of
 // them (on B200 4 / 8 / 12 / 16 windows took a 64 MB y to 3.18 / 2.93 / 2.86 / 2.88 ms end to end; an 8 MB y --
 // one GPU's share of the same vector on eight GPUs -- is quicker in two pieces than in eight, where the seventeen
@@ -873,12 +875,13 @@ static alphasparse_status_t mv_host_pipelined(DeviceCtx *c, T alpha, const T *x,
     // inbound copies start at once, beside whatever is still queued on the library stream (for instance the
     // exchange that is bringing a device x together).
     if (!x_dev) {  // a device x is already where the kernels read it (and ordered on the library stream)
-        ASB_CUDA_OR(cudaMemcpyAsync(c->d_x_stage, x, sizeof(T) * (size_t)c->cols, cudaMemcpyHostToDevice, c->copy_in),
+        ASB_CUDA_OR(copy_to_device(c->d_x_stage, x, sizeof(T) * (size_t)c->cols, c->copy_in),
                     ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
         ASB_CUDA_OR(cudaEventRecord(ev_x, c->copy_in), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
         ASB_CUDA_OR(cudaStreamWaitEvent(st, ev_x, 0), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
 
+    const bool y_pageable = !page_locked(y);
     const int windows = pipeline_windows(sizeof(T) * (size_t)c->rows);
     const int64_t step = ((c->rows + windows - 1) / windows + 1023) & ~1023ll;
     for (int k = 0; k < windows; k++) {
@@ -887,7 +890,7 @@ static alphasparse_status_t mv_host_pipelined(DeviceCtx *c, T alpha, const T *x,
         const RowWindow w{rb, std::min<int64_t>(step, c->rows - rb)};
         cudaEvent_t ev_in = c->ev_pipe[1 + 2 * k], ev_done = c->ev_pipe[2 + 2 * k];
         if (beta != T(0)) {
-            ASB_CUDA_OR(cudaMemcpyAsync(dy + rb, y + rb, sizeof(T) * (size_t)w.count, cudaMemcpyHostToDevice, c->copy_in),
+            ASB_CUDA_OR(copy_to_device(dy + rb, y + rb, sizeof(T) * (size_t)w.count, c->copy_in),
                         ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
             ASB_CUDA_OR(cudaEventRecord(ev_in, c->copy_in), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
             ASB_CUDA_OR(cudaStreamWaitEvent(st, ev_in, 0), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
@@ -895,9 +898,16 @@ static alphasparse_status_t mv_host_pipelined(DeviceCtx *c, T alpha, const T *x,
         s = launch_spmv<T>(c, alpha, dx, beta, dy, st, nullptr, &w);
         if (s != ALPHA_SPARSE_STATUS_SUCCESS) return s;
         ASB_CUDA_OR(cudaEventRecord(ev_done, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+        if (y_pageable) continue;
         ASB_CUDA_OR(cudaStreamWaitEvent(c->copy_out, ev_done, 0), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
         ASB_CUDA_OR(cudaMemcpyAsync(y + rb, dy + rb, sizeof(T) * (size_t)w.count, cudaMemcpyDeviceToHost, c->copy_out),
                     ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    }
+    // Copies into pageable memory keep the host busy, so they start once every window is enqueued.
+    for (int k = 0; y_pageable && k < windows && k * step < c->rows; k++) {
+        const int64_t rb = k * step, count = std::min<int64_t>(step, c->rows - rb);
+        ASB_CUDA_OR(cudaStreamWaitEvent(c->copy_out, c->ev_pipe[2 + 2 * k], 0), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+        ASB_CUDA_OR(copy_to_host(y + rb, dy + rb, sizeof(T) * (size_t)count, c->copy_out), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
     int kernel_status = 0;
     ASB_CUDA_OR(cudaMemcpyAsync(&kernel_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, c->copy_out),
@@ -929,6 +939,64 @@ static alphasparse_status_t select_structured(DeviceCtx *&c, const alphasparse_m
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
+// Host x and y of at most kHostBlockBytes together: both go through one page-locked block.  One copy in; a y of at most
+// kSmallDirectBytes is read and written in the block by the kernel itself, where that is one kernel that touches
+// every y once, else copied back; one wait.  *done: false when no block was to be had.
+// Measured (B200, us a call, copies of pageable memory -> here): fp64 500 / 1,500 (beta != 0) / 10,000 rows of 7 elements
+// 37 / 42 / 56 -> 22 / 25 / 44, fp32 30,000 rows of 20 79 -> 53, power-law fp64 5,000 rows 72 -> 59.
+constexpr size_t kSmallDirectBytes = (size_t)64 << 10;
+
+template <typename T>
+static alphasparse_status_t mv_host_small(DeviceCtx *c, T alpha, const T *x, T beta, T *y, cudaStream_t st, bool *done) {
+    struct Taken {
+        HostBlock b;
+        cudaStream_t st;
+        bool ok, busy = false;
+        ~Taken() {
+            if (busy) (void)cudaStreamSynchronize(st);
+            if (ok) host_block_give(b);
+        }
+    } block{HostBlock{}, st, false};
+    block.ok = host_block_take(&block.b);
+    *done = block.ok;
+    if (!block.ok) return ALPHA_SPARSE_STATUS_SUCCESS;
+    const size_t xb = sizeof(T) * (size_t)c->cols, yb = sizeof(T) * (size_t)c->rows, y_at = (xb + 255) & ~(size_t)255;
+    char *h = static_cast<char *>(block.b.p);
+    int *h_status = reinterpret_cast<int *>(h + kHostBlockBytes - sizeof(int));
+    const bool direct = yb <= kSmallDirectBytes && spmv_one_kernel(c);
+    const bool reports = c->algorithm != ALPHA_SPARSE_CUDA_ALG_VECTOR;  // (the vector kernel has nothing to wait for)
+    alphasparse_status_t s = grow(&c->d_x_stage, &c->x_stage_bytes, y_at + yb, c);
+    if (s != ALPHA_SPARSE_STATUS_SUCCESS) return s;
+    char *d = static_cast<char *>(c->d_x_stage);
+    memcpy(h, x, xb);
+    if (beta != T(0)) memcpy(h + y_at, y, yb);
+    const size_t in = beta != T(0) && !direct ? y_at + yb : xb;
+    T *dy = reinterpret_cast<T *>(d + y_at);
+    if (direct) {
+        void *alias = nullptr;
+        ASB_CUDA_OR(cudaHostGetDevicePointer(&alias, h + y_at, 0), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+        dy = static_cast<T *>(alias);
+    }
+    block.busy = true;
+    if (in > 0) ASB_CUDA_OR(cudaMemcpyAsync(d, h, in, cudaMemcpyHostToDevice, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    s = launch_spmv<T>(c, alpha, reinterpret_cast<const T *>(d), beta, dy, st);
+    if (s != ALPHA_SPARSE_STATUS_SUCCESS) return s;
+    if (!direct)
+        ASB_CUDA_OR(cudaMemcpyAsync(h + y_at, dy, yb, cudaMemcpyDeviceToHost, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    *h_status = 0;
+    if (reports)
+        ASB_CUDA_OR(cudaMemcpyAsync(h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, st),
+                    ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    ASB_CUDA_OR(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    block.busy = false;
+    memcpy(y, h + y_at, yb);
+    if (*h_status != 0) {  // reported once: later calls start clean
+        (void)cudaMemsetAsync(c->d_status, 0, sizeof(int), st);
+        return ALPHA_SPARSE_STATUS_EXECUTION_FAILED;
+    }
+    return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
 // y = alpha * (matrix of c) * x + beta * y with x, y in host or device memory: the part of mv that no longer
 // looks at the handle.  Host vectors are staged (pipelined in row windows when large) and the call returns when
 // y is complete; device vectors are only enqueued.
@@ -943,6 +1011,12 @@ static alphasparse_status_t mv_on_ctx(DeviceCtx *c, T alpha, const T *x, T beta,
     if (!y_dev && c->rows >= kPipelineMinRows && spmv_supports_windows(c) && !c->profile)
         return mv_host_pipelined<T>(c, alpha, x, x_dev, beta, y, st);
 
+    if (!x_dev && !y_dev && sizeof(T) * (size_t)c->cols + sizeof(T) * (size_t)c->rows + 512 <= kHostBlockBytes) {
+        bool done = false;
+        s = mv_host_small<T>(c, alpha, x, beta, y, st, &done);
+        if (done) return s;
+    }
+
     const T *dx = x;
     T *dy = y;
     if (!x_dev) {
@@ -950,7 +1024,7 @@ static alphasparse_status_t mv_on_ctx(DeviceCtx *c, T alpha, const T *x, T beta,
         s = grow(&c->d_x_stage, &c->x_stage_bytes, bytes ? bytes : sizeof(T), c);
         if (s != ALPHA_SPARSE_STATUS_SUCCESS) return s;
         if (bytes)
-            ASB_CUDA_OR(cudaMemcpyAsync(c->d_x_stage, x, bytes, cudaMemcpyHostToDevice, st),
+            ASB_CUDA_OR(copy_to_device(c->d_x_stage, x, bytes, st),
                         ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
         dx = static_cast<const T *>(c->d_x_stage);
     }
@@ -959,7 +1033,7 @@ static alphasparse_status_t mv_on_ctx(DeviceCtx *c, T alpha, const T *x, T beta,
         s = grow(&c->d_y_stage, &c->y_stage_bytes, bytes, c);
         if (s != ALPHA_SPARSE_STATUS_SUCCESS) return s;
         if (beta != T(0))
-            ASB_CUDA_OR(cudaMemcpyAsync(c->d_y_stage, y, bytes, cudaMemcpyHostToDevice, st),
+            ASB_CUDA_OR(copy_to_device(c->d_y_stage, y, bytes, st),
                         ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
         dy = static_cast<T *>(c->d_y_stage);
     }
@@ -977,10 +1051,7 @@ static alphasparse_status_t mv_on_ctx(DeviceCtx *c, T alpha, const T *x, T beta,
     } else {
         s = launch_spmv<T>(c, alpha, dx, beta, dy, st);
         if (s != ALPHA_SPARSE_STATUS_SUCCESS) return s;
-        if (!y_dev) {
-            ASB_CUDA_OR(cudaMemcpyAsync(y, dy, sizeof(T) * (size_t)c->rows, cudaMemcpyDeviceToHost, st),
-                        ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-        }
+        if (!y_dev) ASB_CUDA_OR(copy_to_host(y, dy, sizeof(T) * (size_t)c->rows, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
     if (!y_dev || !x_dev) {
         // a synchronous call can also report a kernel whose bounded wait ran out

@@ -89,6 +89,17 @@ class Download {
     Ring *ring_ = nullptr;
     cudaError_t error_ = cudaSuccess;
 };
+// Device -> host behind the work on `st`; a pageable `dst` is complete on return, a page-locked one once `st` is done.
+cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st);
+bool page_locked(const void *p);  // memory the copy engines reach by themselves (page-locked or device memory)
+// One of a few small page-locked blocks, also addressable by kernels; nothing may be using it when it is given back.
+constexpr size_t kHostBlockBytes = (size_t)512 << 10;
+struct HostBlock {
+    void *p = nullptr;
+    int index = 0;
+};
+bool host_block_take(HostBlock *out);
+void host_block_give(const HostBlock &b);
 // Device memory of conversions, recycled through a small bounded cache.
 struct DeviceBlock {
     void *p = nullptr;
@@ -407,6 +418,8 @@ struct RowWindow {
     int64_t begin, count;
 };
 bool spmv_supports_windows(const DeviceCtx *ctx);
+// A product is one kernel that reads and writes every y once.
+bool spmv_one_kernel(const DeviceCtx *ctx);
 
 template <typename T>
 alphasparse_status_t launch_spmv(DeviceCtx *ctx, T alpha, const T *x, T beta, T *y,

@@ -1169,6 +1169,11 @@ template alphasparse_status_t launch_spmv<float>(DeviceCtx *, float, const float
 template alphasparse_status_t launch_spmv<double>(DeviceCtx *, double, const double *, double,
                                                   double *, cudaStream_t, const PeerPush *, const RowWindow *);
 
+bool spmv_one_kernel(const DeviceCtx *ctx) {
+    return ctx->nnz == 0 || ctx->algorithm == ALPHA_SPARSE_CUDA_ALG_ROWTILE ||
+           (ctx->algorithm == ALPHA_SPARSE_CUDA_ALG_VECTOR && !ctx->mvb.d_split);
+}
+
 bool spmv_supports_windows(const DeviceCtx *ctx) {
     return ctx->nnz > 0 && (ctx->algorithm == ALPHA_SPARSE_CUDA_ALG_VECTOR ||
                             ctx->algorithm == ALPHA_SPARSE_CUDA_ALG_ROWTILE);

@@ -118,7 +118,7 @@ static bool ring_ready(Ring &r) {
     return r.ready = e == cudaSuccess;
 }
 
-static bool page_locked(const void *p) {
+bool page_locked(const void *p) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -175,13 +175,23 @@ cudaError_t copy_to_device_beside(void *dst, const void *src, size_t bytes, cuda
     return e;
 }
 
+cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st) {
+    if (bytes < kRingMinBytes || page_locked(dst)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, st);
+    return Download({{dst, src, bytes}}, st).finish();
+}
+
 Download::Download(std::initializer_list<Piece> pieces, cudaStream_t st) : st_(st) {
     size_t total = 0;
-    for (const Piece &p : pieces) {
-        total += p.bytes;
-        for (size_t off = 0; off < p.bytes; off += kRingChunkBytes)
-            chunks_.push_back({static_cast<char *>(p.dst) + off, static_cast<const char *>(p.src) + off,
-                               std::min(kRingChunkBytes, p.bytes - off)});
+    try {
+        for (const Piece &p : pieces) {
+            total += p.bytes;
+            for (size_t off = 0; off < p.bytes; off += kRingChunkBytes)
+                chunks_.push_back({static_cast<char *>(p.dst) + off, static_cast<const char *>(p.src) + off,
+                                   std::min(kRingChunkBytes, p.bytes - off)});
+        }
+    } catch (...) {  // no memory for the list: nothing is copied, finish() says so
+        error_ = cudaErrorMemoryAllocation;
+        return;
     }
     if (total < kRingMinBytes) return;  // copied by finish()
     Ring *ring = nullptr;
@@ -225,6 +235,40 @@ Download::~Download() {
     if (!ring_) return;
     if (done_ < issued_) (void)cudaStreamSynchronize(st_);  // given up half-way: nothing may still write into the ring
     ring_->mu.unlock();
+}
+
+// ---- small page-locked blocks ---------------------------------------------------------------------------
+//
+// A call with host vectors of a few kilobytes spends its time on copies of pageable memory, each of which the driver
+// stages and waits for by itself.  Such a call packs its vectors into one of these blocks instead: one copy in, results
+// stored or copied straight back into the block, one wait.  Blocks are made on first use and kept, at most
+// kHostBlocks of them (4 MB); a caller that finds none takes the ordinary way.
+
+constexpr int kHostBlocks = 8;
+static std::mutex g_host_block_mu;
+static HostBlock g_host_block[kHostBlocks];
+static bool g_host_block_taken[kHostBlocks];
+
+bool host_block_take(HostBlock *out) {
+    std::lock_guard<std::mutex> lock(g_host_block_mu);
+    for (int k = 0; k < kHostBlocks; k++) {
+        if (g_host_block_taken[k]) continue;
+        HostBlock &b = g_host_block[k];
+        if (!b.p && cudaHostAlloc(&b.p, kHostBlockBytes, cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) {
+            (void)cudaGetLastError();
+            b.p = nullptr;
+            return false;
+        }
+        b.index = k;
+        *out = b;
+        return g_host_block_taken[k] = true;
+    }
+    return false;
+}
+
+void host_block_give(const HostBlock &b) {
+    std::lock_guard<std::mutex> lock(g_host_block_mu);
+    g_host_block_taken[b.index] = false;
 }
 
 // ---- device blocks of assembled matrices ---------------------------------------------------------------
@@ -307,10 +351,11 @@ void device_block_give(DeviceBlock *b) {
     const cudaError_t e = cudaDeviceSynchronize();
     if (prev >= 0 && prev != mine.device) cudaSetDevice(prev);
     std::vector<CacheBlock> out;
-    {
+    bool kept = false;
+    try {
         std::lock_guard<std::mutex> lock(g_cache_mu);
-        if (e == cudaSuccess) g_cache.push_back(mine);
-        else out.push_back(mine);
+        out.reserve(g_cache.size() + 1);  // (this and the next line are all that needs memory)
+        if (e == cudaSuccess) g_cache.push_back(mine), kept = true;
         size_t total = 0;
         for (const CacheBlock &c : g_cache) total += c.bytes;
         while (total > kCacheBytes) {
@@ -318,7 +363,9 @@ void device_block_give(DeviceBlock *b) {
             out.push_back(g_cache.front());
             g_cache.erase(g_cache.begin());
         }
+    } catch (...) {
     }
+    if (!kept) cache_free(mine);
     for (const CacheBlock &c : out) cache_free(c);
 }
 
