@@ -833,9 +833,15 @@ static void launch_row_lanes(DeviceCtx *ctx, T alpha, const T *X, int columns, i
                              int ldy, cudaStream_t st, const RowWindow *w, T *part) {
     // smallest group (4 .. 32 lanes) whose lanes cover the dense columns in one pass, if any
     const int need = (columns + VEC - 1) / VEC;
+    // An X beyond L2 (126 MB) with unstructured columns is read in slices of 256 bytes a row: the part of X in use is half
+    // as large and more of it stays in L2.  Measured (us, 32 -> 16 lanes): 474,552 rows of 27 elements x 128 fp32 / 128 fp64
+    // / 64 fp64 columns 796 / 1639 / 917 -> 721 / 1465 / 852, power-law 400,009 rows x 64 fp64 685 -> 615.  Not where X fits
+    // (50,000 rows x 128 fp64 columns 139 -> 158), neighbouring rows share X rows (stencil 78^3 x 128 fp64 933 -> 1042) or
+    // lanes hold less than 16 bytes (200,000 rows x 127 fp32 columns 603 -> 877).
+    const bool sliced = VEC * sizeof(T) == 16 && ctx->shifted_rows < 0.5 && sizeof(T) * (size_t)ctx->cols * columns > (126u << 20);
     if (need <= 4) launch_row<T, VEC, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
     else if (need <= 8) launch_row<T, VEC, 8>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
-    else if (need <= 16) launch_row<T, VEC, 16>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+    else if (need <= 16 || sliced) launch_row<T, VEC, 16>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
     else launch_row<T, VEC, 32>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
 }
 
