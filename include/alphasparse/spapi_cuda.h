@@ -67,15 +67,18 @@ alphasparse_status_t alphasparse_cuda_set_algorithm(alphasparse_cuda_alg_t alg);
  *                           column block by column block, each block covering at most mv_block_kb (65536) KB of
  *                           x, the first launch applying beta and the later ones adding to y; needs rows in
  *                           ascending column order; 0 = never
- *   spmm_col_via_row (2)    column-major dense blocks of at least this many columns are transposed into row-major copies
+ *   spmm_col_via_row (2)    column-major dense blocks of at least this many columns (of a matrix that is not banded: a
+ *                           lane per row multiplies a banded one as the operands lie) are transposed into row-major copies
  *                           kept with the handle (X, and Y when beta != 0), multiplied by the row-major kernels
  *                           and transposed back: device memory for one more X and Y; 0 = never
  *   spmm_narrow (1)         row-major dense blocks whose rows take at most 32 bytes (8 fp32 / 4 fp64 columns) go through
  *                           a kernel whose lanes split the elements of a sparse row instead of the dense columns
- *   spmm_split_min (1024)   row-major dense-block product on a matrix whose longest row exceeds eight times the mean:
- *                           a row above this many elements is multiplied chunk by chunk (spmm_split_chunk (512)
- *                           elements per chunk, partial sums added in chunk order), so that one lane group does
- *                           not walk a hundred thousand elements alone; 0 = never
+ *   spmm_split_min (1024)   dense-block product of at most 32 bytes a row, or of one column, on a matrix whose longest row
+ *                           exceeds eight times the mean: a row above this many elements is multiplied chunk by chunk
+ *                           (spmm_split_chunk (512) elements per chunk, partial sums added in chunk order), so that
+ *                           one lane group does not walk a hundred thousand elements alone.  Wider row-major
+ *                           blocks cut such a matrix into segments of equal work of at most spmm_split_chunk
+ *                           (and 256) items instead, whatever the value; 0 = neither
  *   spmm_col_blocks (0)     row-major dense-block product in this many column blocks (X slab by slab, Y
  *                           accumulated over the passes); 0 or 1 = one pass, which measured faster on B200
  * Unknown names return ALPHA_SPARSE_STATUS_INVALID_VALUE. */
