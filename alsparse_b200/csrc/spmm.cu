@@ -15,6 +15,7 @@
 #include <limits.h>
 
 #include <algorithm>
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -620,7 +621,7 @@ static alphasparse_status_t spmm_split_prepare(DeviceCtx *ctx, size_t tsz, int c
 // ---- segments of a skewed matrix ---------------------------------------------------------------------
 
 void spmm_segments_destroy(SpmmSegments &s) {
-    cudaFree(s.d_seg), cudaFree(s.d_slot), cudaFree(s.d_row), cudaFree(s.d_first);
+    cudaFree(s.d_seg);  // (one block: the other tables lie behind it)
     for (const SpmmSegments::Part &p : s.parts) cudaFree(p.p);
     s = SpmmSegments{};
 }
@@ -647,12 +648,15 @@ static alphasparse_status_t spmm_segments_ensure(DeviceCtx *ctx, cudaStream_t st
     };
     std::vector<int> slot, first;
     std::vector<MergeCoord> seg;
-    cudaError_t e = device_alloc(&t.d_seg, sizeof(MergeCoord) * ((size_t)t.nseg + 1));
-    if (e == cudaSuccess) e = device_alloc(&t.d_slot, sizeof(int) * (size_t)t.nseg);
+    // one block for the four tables (every segment may leave a part of another row: nseg rows at most), since an
+    // allocation takes as long as everything else here
+    const size_t n = (size_t)t.nseg, table_bytes = sizeof(MergeCoord) * (n + 1) + sizeof(int) * (3 * n + 1);
+    cudaError_t e = device_alloc(&t.d_seg, table_bytes);
     if (e != cudaSuccess) {
         record_cuda_error(e, "segments of the dense-block product");
         return fail(ALPHA_SPARSE_STATUS_ALLOC_FAILED);
     }
+    t.d_slot = reinterpret_cast<int *>(t.d_seg + n + 1), t.d_row = t.d_slot + n, t.d_first = t.d_row + n;
     spmm_segments_kernel<<<(unsigned)(t.nseg / 256 + 1), 256, 0, st>>>((int)ctx->rows, (int)ctx->nnz, ctx->d_row_ptr, (int)items,
                                                                       t.nseg, t.d_seg, t.d_slot);
     count_launch();
@@ -677,9 +681,7 @@ static alphasparse_status_t spmm_segments_ensure(DeviceCtx *ctx, cudaStream_t st
     }
     const size_t ncross = t.cross_row.size();
     if (e == cudaSuccess && ncross > 0) {
-        e = device_alloc(&t.d_row, sizeof(int) * ncross);
-        if (e == cudaSuccess) e = device_alloc(&t.d_first, sizeof(int) * (ncross + 1));
-        if (e == cudaSuccess) e = cudaMemcpyAsync(t.d_row, t.cross_row.data(), sizeof(int) * ncross, cudaMemcpyHostToDevice, st);
+        e = cudaMemcpyAsync(t.d_row, t.cross_row.data(), sizeof(int) * ncross, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(t.d_first, t.cross_first.data(), sizeof(int) * (ncross + 1), cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaMemcpyAsync(t.d_slot, slot.data(), sizeof(int) * slot.size(), cudaMemcpyHostToDevice, st);
@@ -690,8 +692,8 @@ static alphasparse_status_t spmm_segments_ensure(DeviceCtx *ctx, cudaStream_t st
         return fail(e == cudaErrorMemoryAllocation ? ALPHA_SPARSE_STATUS_ALLOC_FAILED : ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
     t.state = 2;
-    sp = t;
-    ctx->device_bytes += (int64_t)(12 * (size_t)t.nseg + 8 * ncross);
+    sp = std::move(t);
+    ctx->device_bytes += (int64_t)table_bytes;
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
