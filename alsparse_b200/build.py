@@ -41,7 +41,7 @@ def nvcc_path():
 
 def build_library(force=False, verbose_ptxas=False):
     srcs = [os.path.join(CSRC, s) for s in CUDA_SOURCES]
-    deps = srcs + [os.path.join(CSRC, "internal.h")] + [
+    deps = srcs + [os.path.join(CSRC, h) for h in ("internal.h", "index_bounds.h")] + [
         os.path.join(ROOT, "include", "alphasparse", h)
         for h in os.listdir(os.path.join(ROOT, "include", "alphasparse"))
     ]

@@ -18,6 +18,7 @@
 #include <utility>
 #include <vector>
 
+#include "index_bounds.h"
 #include "internal.h"
 
 namespace asb {
@@ -189,21 +190,25 @@ __global__ void __launch_bounds__(256, kStreamMinBlocks)
     const T *Xc = X + (live ? c : 0);  // (lanes beyond the last column read the first and drop it)
 
     // ends of rows r .. r + 31 (lane by lane), and of the 32 rows behind them
-    auto load_ends = [&](int from) { return from + lane < r_end ? __ldg(row_ptr + from + lane + 1) : INT_MAX; };
-    int ends = load_ends(r), ends_next = load_ends(r + 32), at = 0;
+    auto load_ends = [&](int ahead) {
+        return ahead_inside(r, ahead + lane, r_end) ? __ldg(row_ptr + ((unsigned)r + ahead + lane + 1)) : INT_MAX;
+    };
+    int ends = load_ends(0), ends_next = load_ends(32), at = 0;
     // Elements of this batch, the next and the one behind it.  Beyond the segment: column 0, which is read and dropped.
     int cj[Q], cn[Q], cm[Q];
     T vj[Q], vn[Q], vm[Q];
-    auto load_batch = [&](int from, int (&cc)[Q], T (&vv)[Q]) {
+    auto load_batch = [&](int from, int ahead, int (&cc)[Q], T (&vv)[Q]) {
 #pragma unroll
         for (int q = 0; q < Q; q++) {
-            const int j = from + q * 32 + lane;
             cc[q] = 0, vv[q] = T(0);
-            if (j < k_end) cc[q] = __ldcs(col + j), vv[q] = __ldcs(val + j);
+            if (ahead_inside(from, ahead + q * 32 + lane, k_end)) {
+                const int j = from + ahead + q * 32 + lane;
+                cc[q] = __ldcs(col + j), vv[q] = __ldcs(val + j);
+            }
         }
     };
-    load_batch(k, cj, vj);
-    load_batch(k + 32 * Q, cn, vn);
+    load_batch(k, 0, cj, vj);
+    load_batch(k, 32 * Q, cn, vn);
     T xv[2][U][VEC];
     auto load_rows = [&](int buf, int group, const int (&cc)[Q]) {  // X rows of the U steps of a group
 #pragma unroll
@@ -246,7 +251,7 @@ __global__ void __launch_bounds__(256, kStreamMinBlocks)
         r++;
         if (++at == 32) {
             at = 0, ends = ends_next;
-            ends_next = load_ends(r + 32);
+            ends_next = load_ends(32);
         }
         row_end = __shfl_sync(0xffffffffu, ends, at);
         fetch_old();
@@ -255,15 +260,15 @@ __global__ void __launch_bounds__(256, kStreamMinBlocks)
     if (k < k_end) load_rows(0, 0, cj);
     while (k < k_end) {  // (everything about k is uniform over the warp)
         const int k0 = k;
-        load_batch(k0 + 64 * Q, cm, vm);
+        load_batch(k0, 64 * Q, cm, vm);
 #pragma unroll
         for (int q = 0; q < Q; q++) vj[q] *= alpha;
 #pragma unroll
         for (int grp = 0; grp < G; grp++) {
             if (grp + 1 < G) load_rows((grp + 1) & 1, grp + 1, cj);
             else load_rows(0, 0, cn);
-            const int kg = k0 + grp * (U * S);
-            if (kg + U * S <= min(row_end, k_end)) {
+            constexpr int GS = U * S;
+            if (ahead_complete(k0, (grp + 1) * GS, min(row_end, k_end))) {
 #pragma unroll
                 for (int u = 0; u < U; u++) {
                     const int e = (grp * U + u) * S;
@@ -271,10 +276,10 @@ __global__ void __launch_bounds__(256, kStreamMinBlocks)
 #pragma unroll
                     for (int i = 0; i < VEC; i++) acc[i] = fma(a, xv[grp & 1][u][i], acc[i]);
                 }
-                k = kg + U * S;
+                k = k0 + (grp + 1) * GS;
                 while (row_end == k) finish_row();
             } else {  // row by row through the group
-                const int stop = min(kg + U * S, k_end);
+                const int stop = ahead_or_end(k0, (grp + 1) * GS, k_end);
                 while (k < stop) {
                     const int hi = min(row_end, stop);
 #pragma unroll
