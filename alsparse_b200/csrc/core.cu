@@ -953,7 +953,7 @@ static alphasparse_status_t mv_host_small(DeviceCtx *c, T alpha, const T *x, T b
         cudaStream_t st;
         bool ok, busy = false;
         ~Taken() {
-            if (busy) (void)cudaStreamSynchronize(st);
+            if (busy && cudaStreamSynchronize(st) != cudaSuccess) (void)cudaGetLastError();
             if (ok) host_block_give(b);
         }
     } block{HostBlock{}, st, false};

@@ -118,6 +118,16 @@ static bool ring_ready(Ring &r) {
     return r.ready = e == cudaSuccess;
 }
 
+// While a stream is being captured nothing of it may pass through a ring: the copy would be recorded, not made, and the
+// chunk's event could not be waited for from then on, by anyone.  The caller then copies directly, and its wait for that
+// copy, which no call here leaves out, ends the capture with an error.
+static bool being_captured(cudaStream_t st) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(st, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
+    (void)cudaGetLastError();  // the legacy stream beside a capturing one
+    return true;
+}
+
 bool page_locked(const void *p) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -130,7 +140,7 @@ bool page_locked(const void *p) {
 cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st) {
     if (bytes == 0) return cudaSuccess;
     Ring *ring = nullptr;
-    if (bytes >= kRingMinBytes && !page_locked(src)) {
+    if (bytes >= kRingMinBytes && !page_locked(src) && !being_captured(st)) {
         cudaError_t e = ring_of_current_device(g_up, &ring);
         if (e != cudaSuccess) return e;
     }
@@ -155,7 +165,7 @@ cudaError_t copy_to_device_beside(void *dst, const void *src, size_t bytes, cuda
     Ring *ring = nullptr;
     cudaError_t e = ring_of_current_device(g_up, &ring);
     if (e != cudaSuccess) return e;
-    if (!ring || bytes < kRingMinBytes) return copy_to_device(dst, src, bytes, st);
+    if (!ring || bytes < kRingMinBytes || being_captured(st)) return copy_to_device(dst, src, bytes, st);
     cudaStream_t side = nullptr;
     cudaEvent_t done = nullptr;
     {
@@ -193,7 +203,7 @@ Download::Download(std::initializer_list<Piece> pieces, cudaStream_t st) : st_(s
         error_ = cudaErrorMemoryAllocation;
         return;
     }
-    if (total < kRingMinBytes) return;  // copied by finish()
+    if (total < kRingMinBytes || being_captured(st)) return;  // copied by finish()
     Ring *ring = nullptr;
     error_ = ring_of_current_device(g_down, &ring);
     if (error_ != cudaSuccess || !ring) return;
@@ -233,7 +243,8 @@ cudaError_t Download::finish() {
 
 Download::~Download() {
     if (!ring_) return;
-    if (done_ < issued_) (void)cudaStreamSynchronize(st_);  // given up half-way: nothing may still write into the ring
+    // given up half-way: nothing may still write into the ring (and no error stays behind for the next call to find)
+    if (done_ < issued_ && cudaStreamSynchronize(st_) != cudaSuccess) (void)cudaGetLastError();
     ring_->mu.unlock();
 }
 
@@ -294,7 +305,7 @@ static void cache_free(const CacheBlock &b) {
     int prev = -1;
     cudaGetDevice(&prev);
     if (prev != b.device) cudaSetDevice(b.device);
-    cudaFree(b.p);
+    if (cudaFree(b.p) != cudaSuccess) (void)cudaGetLastError();
     if (prev >= 0 && prev != b.device) cudaSetDevice(prev);
 }
 
@@ -349,6 +360,7 @@ void device_block_give(DeviceBlock *b) {
     cudaGetDevice(&prev);
     if (prev != mine.device) cudaSetDevice(mine.device);
     const cudaError_t e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) (void)cudaGetLastError();  // (refused inside a capture: the next call is not to find it)
     if (prev >= 0 && prev != mine.device) cudaSetDevice(prev);
     std::vector<CacheBlock> out;
     bool kept = false;
