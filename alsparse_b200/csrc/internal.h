@@ -153,6 +153,8 @@ constexpr size_t kSmemPerSm = 228 * 1024;
 struct DeviceCtx;
 int rowtile_cap(const DeviceCtx *ctx, int tile);
 size_t rowtile_smem_bytes(const DeviceCtx *ctx, int tile);
+// Before a launch of a kernel that stages row tiles with `smem` bytes of dynamic shared memory (at most kRowTileMaxSmem).
+cudaError_t allow_tile_smem(const void *kernel, size_t smem, int device, std::atomic<unsigned long long> *granted);
 
 // Bulk copy global -> shared counted on an mbarrier (shared addresses as 32-bit numbers; both addresses and the size
 // are multiples of 16 bytes), and one poll of the mbarrier.

@@ -1115,11 +1115,15 @@ template <typename T, int KC>
 static alphasparse_status_t launch_col_tile(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y, int ldy,
                                             cudaStream_t st) {
     auto kernel = beta == T(0) ? spmm_col_tile_kernel<T, KC, false> : spmm_col_tile_kernel<T, KC, true>;
+    const size_t smem = rowtile_smem_bytes(ctx, kRowTileSmall);
+    static std::atomic<unsigned long long> granted[2];
+    ASB_CUDA_OR(allow_tile_smem(reinterpret_cast<const void *>(kernel), smem, ctx->device, &granted[beta == T(0) ? 0 : 1]),
+                ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     // A warp does all columns of its rows; where the rows alone do not fill the chip they are shared out.
     const int64_t tiles = (ctx->rows + kRowTileSmall - 1) / kRowTileSmall, chunks = (columns + KC - 1) / KC;
     const int64_t share = std::min(chunks, std::max<int64_t>(1, 148 * 32 / tiles));
     if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
-    kernel<<<dim3((unsigned)tiles, (unsigned)share), kRowTileSmall, rowtile_smem_bytes(ctx, kRowTileSmall), st>>>(
+    kernel<<<dim3((unsigned)tiles, (unsigned)share), kRowTileSmall, smem, st>>>(
         (int)ctx->rows, ctx->d_row_ptr, ctx->d_col, static_cast<const T *>(ctx->d_val), X, columns, ldx, Y, ldy, alpha, beta,
         rowtile_cap(ctx, kRowTileSmall), ctx->d_status);
     if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);

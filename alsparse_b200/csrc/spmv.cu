@@ -681,6 +681,17 @@ size_t rowtile_smem_bytes(const DeviceCtx *ctx, int tile) {
     return (size_t)rowtile_cap(ctx, tile) * (tsz + sizeof(int)) + (tile + 4) * sizeof(int);
 }
 
+// A launch may use 48 KB of shared memory as it is, and that includes what the kernel declares statically (the barrier and
+// flag of stage_row_tile: 128 bytes by -Xptxas -v, taken as 1 KB).  Above, the limit is raised to the most a tile can ask
+// for, once per kernel and device (the limit belongs to both; `granted` holds one bit per device).
+cudaError_t allow_tile_smem(const void *kernel, size_t smem, int device, std::atomic<unsigned long long> *granted) {
+    const unsigned long long bit = device < 64 ? 1ull << device : 0;
+    if (smem + 1024 <= 48 * 1024 || (granted->load(std::memory_order_relaxed) & bit)) return cudaSuccess;
+    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kRowTileMaxSmem);
+    if (e == cudaSuccess) granted->fetch_or(bit, std::memory_order_relaxed);
+    return e;
+}
+
 static int pick_lanes(double mean_quads) {
     // Lanes per row = aligned quads an average row touches, rounded to a power of two.
     int lanes = 1;
@@ -1098,14 +1109,9 @@ static alphasparse_status_t launch_rowtile_as(DeviceCtx *ctx, T alpha, const T *
         spmv_rowtile_kernel<T, TILE, false, false>, spmv_rowtile_kernel<T, TILE, true, false>,
         spmv_rowtile_kernel<T, TILE, false, true>, spmv_rowtile_kernel<T, TILE, true, true>};
     auto kernel = variants[which];
-    // The opt-in limit is a property of the kernel, shared by all handles: only ever raise it.
-    static std::atomic<size_t> granted[4] = {{0}, {0}, {0}, {0}};
-    if (smem > 48 * 1024 && granted[which].load() < smem) {
-        ASB_CUDA_OR(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)kRowTileMaxSmem),
-                    ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-        granted[which].store(kRowTileMaxSmem);
-    }
+    static std::atomic<unsigned long long> granted[4];
+    ASB_CUDA_OR(allow_tile_smem(reinterpret_cast<const void *>(kernel), smem, ctx->device, &granted[which]),
+                ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
     // w.begin is a multiple of kRowTile (the caller's duty): tiles, and the 16-byte alignment of the
     // offset copies, are the same as in a full launch
