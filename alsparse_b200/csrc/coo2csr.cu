@@ -307,10 +307,13 @@ static alphasparse_status_t radix_sort(const SortScratch<K> &s, long long n, int
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
-// One scratch block per conversion, given back when it goes out of scope.
+// One block of a conversion, used on the library stream alone and given back when it goes out of scope.
 struct ScopedBlock {
     DeviceBlock b;
-    ~ScopedBlock() { device_block_give(&b); }
+    BlockUse use;
+    explicit ScopedBlock(cudaStream_t st) { use.add(st); }
+    ~ScopedBlock() { device_block_give(&b, use); }
+    void done() { use = BlockUse{}; }  // the stream has been waited for
 };
 
 // Host COO arrays in, device CSR (one block, ctx_adopt_block's layout) and HOST 3-array CSR out (caller-provided buffers
@@ -321,7 +324,7 @@ template <typename T, typename K>
 static alphasparse_status_t coo_to_csr_keyed(int64_t rows, int64_t cols, int64_t nnz, const int *ri, const int *ci,
                                              const T *v, int *out_ptr, int *out_col, T *out_val, DeviceBlock *out) {
     cudaStream_t st = current_stream();
-    ScopedBlock scratch, result;
+    ScopedBlock scratch(st), result(st);
     const size_t n = (size_t)nnz;
 #define TRY(expr, code) ASB_CUDA_OR(expr, code)
     auto layout = [&](void *p, int **d_ri, int **d_ci, T **d_v, unsigned long long **d_bad) {
@@ -333,9 +336,9 @@ static alphasparse_status_t coo_to_csr_keyed(int64_t rows, int64_t cols, int64_t
     int *d_ri, *d_ci;
     T *d_v;
     unsigned long long *d_bad;
-    TRY(device_block_take(layout(nullptr, &d_ri, &d_ci, &d_v, &d_bad).second, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    TRY(device_block_take(layout(nullptr, &d_ri, &d_ci, &d_v, &d_bad).second, st, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
     const SortScratch<K> sort = layout(scratch.b.p, &d_ri, &d_ci, &d_v, &d_bad).first;
-    TRY(device_block_take(adopt_block_bytes(sizeof(T), rows, nnz), &result.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    TRY(device_block_take(adopt_block_bytes(sizeof(T), rows, nnz), st, &result.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
     int *d_ptr, *d_col;
     T *d_val;
     adopt_block_layout(result.b.p, rows, nnz, &d_ptr, &d_col, &d_val);
@@ -367,6 +370,7 @@ static alphasparse_status_t coo_to_csr_keyed(int64_t rows, int64_t cols, int64_t
                    {&bad, d_bad, 8}},
                   st);
     TRY(back.finish(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    scratch.done(), result.done();
     if (bad) return ALPHA_SPARSE_STATUS_INVALID_VALUE;
     *out = result.b;
     result.b = DeviceBlock{};
@@ -424,7 +428,7 @@ template <typename T>
 alphasparse_status_t transpose_csr_device(const DeviceCtx *c, int **out_ptr, int **out_col, T **out_val) {
     cudaStream_t st = current_stream();
     const int64_t nnz = c->nnz, rows = c->rows, cols = c->cols;
-    ScopedBlock scratch;
+    ScopedBlock scratch(st);
     int *tptr = nullptr, *tcol = nullptr;
     T *tval = nullptr;
     auto release = [&] { cudaFree(tptr), cudaFree(tcol), cudaFree(tval); };
@@ -448,7 +452,7 @@ alphasparse_status_t transpose_csr_device(const DeviceCtx *c, int **out_ptr, int
     if (nnz > 0) {
         Carve need(nullptr);
         (void)SortScratch<unsigned>(need, nnz);
-        TRY(device_block_take(need.used, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+        TRY(device_block_take(need.used, st, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
         Carve have(scratch.b.p);
         const SortScratch<unsigned> sort(have, nnz);
         TRY(cudaMemcpyAsync(sort.keys[0], c->d_col, sizeof(int) * n, cudaMemcpyDeviceToDevice, st),
@@ -467,6 +471,7 @@ alphasparse_status_t transpose_csr_device(const DeviceCtx *c, int **out_ptr, int
         TRY(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
     TRY(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    scratch.done();
 #undef TRY
     *out_ptr = tptr, *out_col = tcol, *out_val = tval;
     return ALPHA_SPARSE_STATUS_SUCCESS;
@@ -583,7 +588,7 @@ alphasparse_status_t derive_csr_device(const DeviceCtx *c, int type, int upper, 
     cudaStream_t st = current_stream();
     const int64_t nnz = c->nnz, rows = c->rows;
     const DeriveRule rule{type, upper, unit, flip, diag_rule};
-    ScopedBlock scratch;
+    ScopedBlock scratch(st);
     unsigned *d_sums = nullptr, *d_count = nullptr;
     int *d_pick = nullptr, *dptr = nullptr, *dcol = nullptr;
     T *dval = nullptr;
@@ -647,7 +652,7 @@ alphasparse_status_t derive_csr_device(const DeviceCtx *c, int type, int upper, 
     if (m > 0) {
         Carve need(nullptr);
         (void)SortScratch<unsigned long long>(need, m);
-        TRY(device_block_take(need.used, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+        TRY(device_block_take(need.used, st, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
         Carve have(scratch.b.p);
         const SortScratch<unsigned long long> sort(have, m);
         const int bits = bits_for(rows);  // square: rows == cols
@@ -668,6 +673,7 @@ alphasparse_status_t derive_csr_device(const DeviceCtx *c, int type, int upper, 
         TRY(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
     TRY(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    scratch.done();
 #undef TRY
     release(false);
     *out_ptr = dptr, *out_col = dcol, *out_val = dval, *out_nnz = m;

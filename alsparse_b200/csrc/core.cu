@@ -136,7 +136,7 @@ void ctx_destroy(DeviceCtx *c) {
     cudaGetDevice(&prev);
     cudaSetDevice(c->device);
     if (c->block.p) {
-        device_block_give(&c->block);
+        device_block_give(&c->block, c->block_use);
     } else {
         cudaFree(c->d_row_ptr);
         cudaFree(c->d_col);
@@ -287,7 +287,7 @@ alphasparse_status_t ctx_adopt_block(int datatype, int64_t rows, int64_t cols, i
     *out = nullptr;
     DeviceCtx *c = new (std::nothrow) DeviceCtx();
     if (!c) {
-        device_block_give(block);
+        device_block_give(block, BlockUse{});
         return ALPHA_SPARSE_STATUS_ALLOC_FAILED;
     }
     const size_t tsz = datatype == ALPHA_SPARSE_DATATYPE_DOUBLE ? 8 : 4;
@@ -299,6 +299,7 @@ alphasparse_status_t ctx_adopt_block(int datatype, int64_t rows, int64_t cols, i
     c->d_row_ptr = reinterpret_cast<int *>(p), c->d_col = reinterpret_cast<int *>(p + l.col), c->d_val = p + l.val;
     c->d_status = reinterpret_cast<int *>(p + l.status), c->d_stats = reinterpret_cast<unsigned long long *>(p + l.stats);
     c->device_bytes = (int64_t)l.bytes;
+    block_used(c, current_stream());
     cudaError_t e = cudaMemsetAsync(c->d_status, 0, sizeof(int), current_stream());
     alphasparse_status_t s = ALPHA_SPARSE_STATUS_EXECUTION_FAILED;
     if (e == cudaSuccess) {
@@ -381,7 +382,7 @@ static alphasparse_status_t finish_csr_handle(alphasparse_matrix_t *A, int64_t r
     M *m = static_cast<M *>(calloc(1, sizeof(M)));
     if (!h || !m) {
         free(h), free(m), free(ptr), free(col), free(val);
-        if (on_device) device_block_give(on_device);
+        if (on_device) device_block_give(on_device, BlockUse{});
         return ALPHA_SPARSE_STATUS_ALLOC_FAILED;
     }
     m->values = val;
@@ -1691,6 +1692,8 @@ alphasparse_status_t alphasparse_cuda_get_device_csr(const alphasparse_matrix_t 
                                                      ALPHA_INT **d_col_indx, void **d_values) {
     DeviceCtx *c = ctx_of(A);
     if (!c) return ALPHA_SPARSE_STATUS_INVALID_HANDLE;
+    std::lock_guard<std::mutex> lock(c->mu);
+    c->block_use.where = BlockUse::kAnywhere;  // (by the caller's own kernels)
     if (d_row_ptr) *d_row_ptr = c->d_row_ptr;
     if (d_col_indx) *d_col_indx = c->d_col;
     if (d_values) *d_values = c->d_val;

@@ -91,6 +91,7 @@ class Download {
 };
 // Device -> host behind the work on `st`; a pageable `dst` is complete on return, a page-locked one once `st` is done.
 cudaError_t copy_to_host(void *dst, const void *src, size_t bytes, cudaStream_t st);
+bool being_captured(cudaStream_t st);
 bool page_locked(const void *p);  // memory the copy engines reach by themselves (page-locked or device memory)
 // One of a few small page-locked blocks, also addressable by kernels; nothing may be using it when it is given back.
 constexpr size_t kHostBlockBytes = (size_t)512 << 10;
@@ -106,8 +107,14 @@ struct DeviceBlock {
     size_t bytes = 0;
     int device = 0;
 };
-cudaError_t device_block_take(size_t bytes, DeviceBlock *out);
-void device_block_give(DeviceBlock *b);  // waits until the device is idle
+// Where work that touches a block has been queued: nowhere (or it is done), on one stream, or beyond what can be told.
+struct BlockUse {
+    enum { kNowhere, kOneStream, kAnywhere } where = kNowhere;
+    unsigned long long stream = 0;  // its number: never used twice, as an address may be
+    void add(cudaStream_t st);      // work is about to be queued on `st`
+};
+cudaError_t device_block_take(size_t bytes, cudaStream_t st, DeviceBlock *out);  // for use on `st` first of all
+void device_block_give(DeviceBlock *b, const BlockUse &use);
 bool device_cache_trim();                // gives everything cached back to CUDA; true if there was anything
 bool device_alloc_denied();              // counts an allocation for alphasparse_cuda_debug_fail_alloc; true: it is to fail
 
@@ -367,6 +374,7 @@ struct DeviceCtx {
     unsigned *d_chunk_done = nullptr;  // per chunk of kPushChunkTiles tiles (exchange calls only)
 
     DeviceBlock block;                       // holds d_row_ptr .. d_val, d_status and d_stats when it is set
+    BlockUse block_use;
     unsigned long long *d_stats = nullptr;  // counters of the analysis (kept: allocations are what creation waits for)
     int *d_status = nullptr;  // error word set by kernels whose bounded waits ran out (0 = fine)
 
@@ -394,6 +402,9 @@ struct DeviceCtx {
 };
 
 DeviceCtx *ctx_of(const alphasparse_matrix_t A);
+inline void block_used(DeviceCtx *ctx, cudaStream_t st) {  // work on the matrix is about to be queued on `st`
+    if (ctx->block.p) ctx->block_use.add(st);
+}
 
 // Upload + analysis.  `ptr` has rows+1 zero-based offsets.  On failure everything allocated
 // so far is released and *out stays null.

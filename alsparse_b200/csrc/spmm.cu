@@ -925,6 +925,7 @@ template <typename T>
 alphasparse_status_t launch_spmm_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx,
                                      T beta, T *Y, int ldy, cudaStream_t st, const RowWindow *w) {
     if (ctx->rows == 0 || columns <= 0 || (w && w->count <= 0)) return ALPHA_SPARSE_STATUS_SUCCESS;
+    block_used(ctx, st);
     const bool narrow = (size_t)columns * sizeof(T) <= 32 && option(kOptSpmmNarrow);
     T *part = nullptr;
     alphasparse_status_t bs = narrow ? spmm_split_prepare(ctx, sizeof(T), columns, st) : spmm_segments_prepare<T>(ctx, columns, st, &part);
@@ -1181,6 +1182,7 @@ template <typename T>
 alphasparse_status_t launch_spmm_col(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
                                      int ldy, cudaStream_t st) {
     if (ctx->rows == 0 || columns <= 0) return ALPHA_SPARSE_STATUS_SUCCESS;
+    block_used(ctx, st);
     if (ctx->algorithm == ALPHA_SPARSE_CUDA_ALG_ROWTILE && ctx->shifted_rows >= 0.5 && ctx->nnz > 0 &&
         rowtile_smem_bytes(ctx, kRowTileSmall) <= 48 * 1024) {
         const int passes = (columns + 7) / 8, per = (columns + passes - 1) / passes;  // columns in equal groups of at most 8

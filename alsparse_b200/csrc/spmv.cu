@@ -882,6 +882,7 @@ static alphasparse_status_t build_merge_tables(DeviceCtx *ctx, cudaStream_t st) 
 
 alphasparse_status_t ctx_analyse(DeviceCtx *ctx) {
     cudaStream_t st = current_stream();
+    block_used(ctx, st);
     ctx->algorithm = ALPHA_SPARSE_CUDA_ALG_VECTOR;
     ctx->lanes = 4;
     ctx->max_row_nnz = 0, ctx->empty_rows = ctx->rows, ctx->mean_row_nnz = 0.0;
@@ -1135,6 +1136,7 @@ template <typename T>
 alphasparse_status_t launch_spmv(DeviceCtx *ctx, T alpha, const T *x, T beta, T *y,
                                  cudaStream_t st, const PeerPush *push, const RowWindow *window) {
     if (ctx->rows == 0) return ALPHA_SPARSE_STATUS_SUCCESS;
+    block_used(ctx, st);
     const RowWindow w = window ? *window : RowWindow{0, ctx->rows};
     if (window && (push || !spmv_supports_windows(ctx))) return ALPHA_SPARSE_STATUS_INTERNAL_ERROR;
     bool pushed = false;  // whether the kernel's own epilogue delivered y to the peers

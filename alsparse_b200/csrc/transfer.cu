@@ -121,7 +121,7 @@ static bool ring_ready(Ring &r) {
 // While a stream is being captured nothing of it may pass through a ring: the copy would be recorded, not made, and the
 // chunk's event could not be waited for from then on, by anyone.  The caller then copies directly, and its wait for that
 // copy, which no call here leaves out, ends the capture with an error.
-static bool being_captured(cudaStream_t st) {
+bool being_captured(cudaStream_t st) {
     cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &status) == cudaSuccess) return status != cudaStreamCaptureStatusNone;
     (void)cudaGetLastError();  // the legacy stream beside a capturing one
@@ -178,9 +178,13 @@ cudaError_t copy_to_device_beside(void *dst, const void *src, size_t bytes, cuda
         side = ring->side, done = ring->side_done;
     }
     e = copy_to_device(dst, src, bytes, side);
+    if (e != cudaSuccess) {  // nothing may be on its way to `dst` when the caller gives it up
+        if (cudaStreamSynchronize(side) != cudaSuccess) (void)cudaGetLastError();
+        return e;
+    }
     // (two threads may record one after the other: both copies are then in front of the later record, and the earlier
     // waiter waits for at least its own)
-    if (e == cudaSuccess) e = cudaEventRecord(done, side);
+    e = cudaEventRecord(done, side);
     if (e == cudaSuccess) e = cudaStreamWaitEvent(st, done, 0);
     return e;
 }
@@ -287,8 +291,12 @@ void host_block_give(const HostBlock &b) {
 // Converting triples needs scratch for the sort and one block for the resulting arrays.  A program that assembles its
 // matrix at every step would pay cudaMalloc and cudaFree for both each time (1-6 ms of a 5 ms conversion), so blocks
 // given back here are kept for the next conversion: at most kCacheBytes over all devices, the oldest leave first, and
-// all of them when an allocation fails.  A block is idle when it enters (the giver waits for the device, as cudaFree
-// does), so it can be used on any stream by any thread.
+// all of them when an allocation fails.
+//
+// A handle may be destroyed while products with it are still queued.  Nothing is waited for then: waiting for the device
+// would end every capture in progress in the process with an error, whoever is recording it, and the stream of the
+// products may be gone.  A block whose work was all queued on one stream goes out again only to a taker on that stream,
+// which waits for it; one that cannot be told is given to CUDA, which waits for everything.
 
 constexpr size_t kCacheBytes = (size_t)512 << 20;
 constexpr size_t kCacheGrain = (size_t)256 << 10;
@@ -297,6 +305,7 @@ struct CacheBlock {
     void *p;
     size_t bytes;
     int device;
+    BlockUse use;  // kNowhere or kOneStream
 };
 static std::mutex g_cache_mu;
 static std::vector<CacheBlock> g_cache;  // oldest first
@@ -319,25 +328,53 @@ bool device_cache_trim() {
     return !out.empty();
 }
 
-cudaError_t device_block_take(size_t bytes, DeviceBlock *out) {
+static bool stream_number(cudaStream_t st, unsigned long long *number) {
+    if (being_captured(st)) return false;  // (a graph runs where it is launched)
+    if (cudaStreamGetId(st, number) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
+void BlockUse::add(cudaStream_t st) {
+    unsigned long long number = 0;
+    if (where == kAnywhere) return;
+    if (!stream_number(st, &number) || (where == kOneStream && number != stream)) where = kAnywhere;
+    else where = kOneStream, stream = number;
+}
+
+cudaError_t device_block_take(size_t bytes, cudaStream_t st, DeviceBlock *out) {
     *out = DeviceBlock{};
     const size_t want = (std::max<size_t>(bytes, 1) + kCacheGrain - 1) / kCacheGrain * kCacheGrain;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
     if (device_alloc_denied()) return cudaErrorMemoryAllocation;
+    unsigned long long number = 0;
+    const bool numbered = stream_number(st, &number);
+    bool wait = false;
     {
         std::lock_guard<std::mutex> lock(g_cache_mu);
         size_t best = g_cache.size();
-        for (size_t i = 0; i < g_cache.size(); i++)
-            if (g_cache[i].device == dev && g_cache[i].bytes >= want && g_cache[i].bytes <= 2 * want &&
-                (best == g_cache.size() || g_cache[i].bytes < g_cache[best].bytes))
-                best = i;
+        for (size_t i = 0; i < g_cache.size(); i++) {
+            const CacheBlock &c = g_cache[i];
+            if (c.device != dev || c.bytes < want || c.bytes > 2 * want) continue;
+            if (c.use.where != BlockUse::kNowhere && !(numbered && c.use.stream == number)) continue;
+            if (best == g_cache.size() || c.bytes < g_cache[best].bytes) best = i;
+        }
         if (best < g_cache.size()) {
             out->p = g_cache[best].p, out->bytes = g_cache[best].bytes, out->device = dev;
+            wait = g_cache[best].use.where != BlockUse::kNowhere;
             g_cache.erase(g_cache.begin() + (ptrdiff_t)best);
-            return cudaSuccess;
         }
+    }
+    if (out->p) {
+        e = wait ? cudaStreamSynchronize(st) : cudaSuccess;
+        if (e != cudaSuccess) {
+            BlockUse use;
+            use.where = BlockUse::kAnywhere;
+            device_block_give(out, use);
+        }
+        return e;
     }
     e = cudaMalloc(&out->p, want);
     if (e == cudaErrorMemoryAllocation && device_cache_trim()) {
@@ -348,26 +385,20 @@ cudaError_t device_block_take(size_t bytes, DeviceBlock *out) {
     return e;
 }
 
-void device_block_give(DeviceBlock *b) {
+void device_block_give(DeviceBlock *b, const BlockUse &use) {
     if (!b->p) return;
-    const CacheBlock mine{b->p, b->bytes, b->device};
+    const CacheBlock mine{b->p, b->bytes, b->device, use};
     *b = DeviceBlock{};
-    if (mine.bytes > kCacheBytes / 2) {
+    if (mine.bytes > kCacheBytes / 2 || use.where == BlockUse::kAnywhere) {
         cache_free(mine);
         return;
     }
-    int prev = -1;
-    cudaGetDevice(&prev);
-    if (prev != mine.device) cudaSetDevice(mine.device);
-    const cudaError_t e = cudaDeviceSynchronize();
-    if (e != cudaSuccess) (void)cudaGetLastError();  // (refused inside a capture: the next call is not to find it)
-    if (prev >= 0 && prev != mine.device) cudaSetDevice(prev);
     std::vector<CacheBlock> out;
     bool kept = false;
     try {
         std::lock_guard<std::mutex> lock(g_cache_mu);
         out.reserve(g_cache.size() + 1);  // (this and the next line are all that needs memory)
-        if (e == cudaSuccess) g_cache.push_back(mine), kept = true;
+        g_cache.push_back(mine), kept = true;
         size_t total = 0;
         for (const CacheBlock &c : g_cache) total += c.bytes;
         while (total > kCacheBytes) {

@@ -1,5 +1,6 @@
-"""Copies between pageable host memory and the device through the page-locked rings: what else the process is doing."""
+"""Page-locked rings and recycled device blocks: what else the process is doing meanwhile."""
 import ctypes as C
+import threading
 
 import numpy as np
 import pytest
@@ -60,3 +61,74 @@ def test_copies_refused_inside_a_capture_leave_later_ones_alone():
     assert status == capi.SUCCESS, spblas.last_error()
     for h in (coo, B):
         spblas.destroy(h)
+
+
+@pytest.mark.parametrize("mode", [1, 2])  # thread-local, relaxed: what other threads do is no part of the capture
+def test_assembly_in_another_thread_leaves_a_capture_alone(mode):
+    """A program that records a graph in one thread and converts and destroys matrices in another."""
+    ri, ci, v = triples(300000, 20000)
+
+    def assemble():
+        st, coo = spblas.create_coo("d", capi.BASE_ZERO, 20000, 20000, len(v), ri, ci, v)
+        st2, A = spblas.convert_csr(coo)
+        assert st == st2 == capi.SUCCESS, spblas.last_error()
+        spblas.destroy(coo)
+        return A
+
+    handles = [assemble() for _ in range(3)]
+    cu, stream, done = C.CDLL("libcuda.so.1"), torch.cuda.Stream(), []
+    x, y = torch.ones(20000, dtype=torch.float64, device="cuda"), torch.zeros(20000, dtype=torch.float64, device="cuda")
+    assert spblas.mv("d", 0, 1.0, handles[1], spblas.descr(), x, 0.0, y) == capi.SUCCESS  # queued, not waited for
+    assert cu.cuStreamBeginCapture_v2(C.c_void_p(stream.cuda_stream), mode) == 0
+
+    def work():
+        torch.cuda.set_device(0)
+        for A in handles:
+            spblas.destroy(A)
+        spblas.destroy(assemble())
+        done.append(True)
+
+    t = threading.Thread(target=work)
+    t.start()
+    t.join()
+    graph = C.c_void_p()
+    ended = cu.cuStreamEndCapture(C.c_void_p(stream.cuda_stream), C.byref(graph))
+    if graph.value:
+        cu.cuGraphDestroy(graph)
+    assert done and ended == 0
+
+
+def test_memory_of_a_destroyed_handle_is_not_handed_out_under_its_products():
+    """A product still queued when its handle is destroyed, and a conversion of the same size right behind it."""
+    ri, ci, v = triples(300000, 20000)
+
+    def assemble(values):
+        st, coo = spblas.create_coo("d", capi.BASE_ZERO, 20000, 20000, len(v), ri, ci, values)
+        st2, A = spblas.convert_csr(coo)
+        assert st == st2 == capi.SUCCESS, spblas.last_error()
+        spblas.destroy(coo)
+        return A
+
+    x = torch.ones(20000, dtype=torch.float64, device="cuda")
+    want, got = (torch.zeros(20000, dtype=torch.float64, device="cuda") for _ in range(2))
+    side = torch.cuda.Stream()
+    A = assemble(v)
+    assert spblas.mv("d", 0, 1.0, A, spblas.descr(), x, 0.0, want) == capi.SUCCESS
+    torch.cuda.synchronize()
+    for stream in (None, side.cuda_stream):
+        got.zero_()
+        torch.cuda.synchronize()
+        spblas.set_stream(stream)
+        try:
+            with torch.cuda.stream(side if stream else torch.cuda.default_stream()):
+                torch.cuda._sleep(100_000_000)  # about 50 ms in front of the product
+                assert spblas.mv("d", 0, 1.0, A, spblas.descr(), x, 0.0, got) == capi.SUCCESS
+        finally:
+            spblas.set_stream(None)
+        spblas.destroy(A)
+        A = assemble(-v)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+        spblas.destroy(A)
+        A = assemble(v)
+    spblas.destroy(A)
