@@ -60,19 +60,24 @@ static void copy_streaming(char *dst, const char *src, size_t bytes) {
     _mm_sfence();
 }
 
-// memcpy by all cores once the piece is worth waking them for
+// memcpy by all cores once the piece is worth waking them for.  The team is always the whole one, of which a smaller
+// piece gives work to a few: a region that asks for fewer threads than the last one makes the OpenMP runtime end the
+// others, and the next large piece starts them anew (190-550 us for a 4 MB piece that takes 30; a pageable y of 8.8 MB,
+// with a smaller last piece in every call, took 1.3 ms instead of 0.6).
 void host_copy(void *dst, const void *src, size_t bytes) {
     constexpr size_t kPerThread = 128 << 10;
-    const int threads = (int)std::min<size_t>((size_t)std::max(1, omp_get_max_threads()), bytes / kPerThread);
-    if (threads <= 1) {
+    const size_t pieces = std::min<size_t>((size_t)std::max(1, omp_get_max_threads()), bytes / kPerThread);
+    if (pieces <= 1) {
         memcpy(dst, src, bytes);
         return;
     }
-#pragma omp parallel num_threads(threads)
+#pragma omp parallel
     {
-        const size_t t = (size_t)omp_get_thread_num(), nt = (size_t)omp_get_num_threads();
-        const size_t a = (bytes * t / nt) & ~(size_t)63, e = t + 1 == nt ? bytes : (bytes * (t + 1) / nt) & ~(size_t)63;
-        copy_streaming(static_cast<char *>(dst) + a, static_cast<const char *>(src) + a, e - a);
+        const size_t t = (size_t)omp_get_thread_num(), n = std::min(pieces, (size_t)omp_get_num_threads());
+        if (t < n) {
+            const size_t a = (bytes * t / n) & ~(size_t)63, e = t + 1 == n ? bytes : (bytes * (t + 1) / n) & ~(size_t)63;
+            copy_streaming(static_cast<char *>(dst) + a, static_cast<const char *>(src) + a, e - a);
+        }
     }
 }
 
