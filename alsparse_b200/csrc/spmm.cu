@@ -539,14 +539,20 @@ __global__ void spmm_long_reduce_kernel(const int *__restrict__ long_row, const 
     }
 }
 
+// Rows that one lane group would still be walking long after every other row is done.  (Only where the rows are uneven:
+// rows that are all long keep every lane group equally busy as they are.)
+static bool spmm_long_rows(const DeviceCtx *ctx) {
+    const int64_t min_len = option(kOptSpmmSplitMin);
+    return min_len > 0 && ctx->max_row_nnz > min_len && (double)ctx->max_row_nnz > 8.0 * ctx->mean_row_nnz;
+}
+
 // Looks at the row lengths once (first row-major product of the handle) and builds the chunk tables when some row
 // is longer than spmm_split_min.
 static alphasparse_status_t spmm_split_ensure(DeviceCtx *ctx, cudaStream_t st) {
     SpmmSplit &sp = ctx->split;
     if (sp.state != 0) return ALPHA_SPARSE_STATUS_SUCCESS;
     const int64_t min_len = option(kOptSpmmSplitMin), chunk = std::max<int64_t>(64, option(kOptSpmmSplitChunk));
-    // (only where the rows are uneven: rows that are all long keep every lane group equally busy as they are)
-    if (min_len <= 0 || ctx->max_row_nnz <= min_len || ctx->rows == 0 || (double)ctx->max_row_nnz <= 8.0 * ctx->mean_row_nnz) {
+    if (ctx->rows == 0 || !spmm_long_rows(ctx)) {
         sp.state = 1;
         return ALPHA_SPARSE_STATUS_SUCCESS;
     }
@@ -752,8 +758,9 @@ static alphasparse_status_t spmm_segments_prepare(DeviceCtx *ctx, int columns, c
 // blocks.  Blocking does take the reads of X off HBM, but every stored element still pulls a whole row of X from
 // L2 into an SM, and that stream (17 GB) already runs at the pace the one-pass kernel reaches from HBM; the
 // extra passes over Y and the shorter per-row runs only add to it.
-static int spmm_pick_blocks(const DeviceCtx *, size_t) {
-    const int64_t blocks = option(kOptSpmmColBlocks);
+// Rows too long for one lane group come first: with them the product runs in segments, in one pass.
+static int spmm_pick_blocks(const DeviceCtx *ctx) {
+    const int64_t blocks = spmm_long_rows(ctx) ? 1 : option(kOptSpmmColBlocks);
     return (int)std::max<int64_t>(1, std::min<int64_t>(blocks, 64));
 }
 
@@ -787,7 +794,7 @@ static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx
                        int ldy, cudaStream_t st, const RowWindow *w, T *part) {
     SpmmSegments &sp = ctx->segments;
     if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
-    if (!part && ctx->spmm.d_split) {
+    if (ctx->spmm.d_split) {
         launch_row_blocks<T, VEC, LPR>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
         if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
         return;
@@ -928,15 +935,17 @@ alphasparse_status_t launch_spmm_row(DeviceCtx *ctx, T alpha, const T *X, int co
     block_used(ctx, st);
     const bool narrow = (size_t)columns * sizeof(T) <= 32 && option(kOptSpmmNarrow);
     T *part = nullptr;
-    alphasparse_status_t bs = narrow ? spmm_split_prepare(ctx, sizeof(T), columns, st) : spmm_segments_prepare<T>(ctx, columns, st, &part);
-    if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
-    bs = col_blocks_ensure(ctx, ctx->spmm, spmm_pick_blocks(ctx, sizeof(T) * (size_t)ctx->cols * (size_t)ldx), st);
-    if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
+    alphasparse_status_t bs;
     if (narrow) {
+        bs = spmm_split_prepare(ctx, sizeof(T), columns, st);
+        if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
         launch_narrow<T>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
         ASB_CUDA_OR(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
         return ALPHA_SPARSE_STATUS_SUCCESS;
     }
+    bs = col_blocks_ensure(ctx, ctx->spmm, spmm_pick_blocks(ctx), st);
+    if (bs == ALPHA_SPARSE_STATUS_SUCCESS && !ctx->spmm.d_split) bs = spmm_segments_prepare<T>(ctx, columns, st, &part);
+    if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
     auto fits = [&](int vec) {
         const uintptr_t mask = (uintptr_t)(vec * sizeof(T) - 1);
         return columns % vec == 0 && ldx % vec == 0 && ldy % vec == 0 &&

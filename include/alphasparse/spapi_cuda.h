@@ -79,8 +79,9 @@ alphasparse_status_t alphasparse_cuda_set_algorithm(alphasparse_cuda_alg_t alg);
  *                           one lane group does not walk a hundred thousand elements alone.  Wider row-major
  *                           blocks cut such a matrix into segments of equal work of at most spmm_split_chunk
  *                           (and 256) items instead, whatever the value; 0 = neither
- *   spmm_col_blocks (0)     row-major dense-block product in this many column blocks (X slab by slab, Y
- *                           accumulated over the passes); 0 or 1 = one pass, which measured faster on B200
+ *   spmm_col_blocks (0)     row-major dense-block product of more than 32 bytes a row in this many column blocks (X slab
+ *                           by slab, Y accumulated over the passes), except on a matrix that spmm_split_min applies
+ *                           to; 0 or 1 = one pass, which measured faster on B200
  * Unknown names return ALPHA_SPARSE_STATUS_INVALID_VALUE. */
 alphasparse_status_t alphasparse_cuda_set_option(const char *name, int64_t value);
 alphasparse_status_t alphasparse_cuda_get_option(const char *name, int64_t *value);

@@ -133,3 +133,26 @@ def test_products_that_may_not_allocate(kind):
         spblas.set_stream(None)
     assert torch.equal(y, want)
     spblas.destroy(A)
+
+
+@pytest.mark.parametrize("longest,blocks_run", [(90, True), (900, True), (1500, False)])
+def test_column_blocks_where_they_are_asked_for(longest, blocks_run):
+    """Mean 12: even rows, a row that the segment table would cut, and one too long for a lane group (one pass then)."""
+    lens = synth.rowlen_poisson(13, 4000, 12.0, 60).copy()
+    lens[11] = longest
+    m = synth.from_lengths("s", 13, lens, 3000)
+    A = make_handle("s", m)
+    try:
+        for blocks in (2, 5, 1):
+            assert spblas.set_option("spmm_col_blocks", blocks) == capi.SUCCESS
+            check("s", m, A, 24)  # (the table)
+            before = spblas.launch_count()
+            check("s", m, A, 24)
+            launches, reported = spblas.launch_count() - before, spblas.mat_info(A)[1].spmm_col_blocks
+            if blocks_run and blocks > 1:
+                assert launches == blocks and reported == blocks
+            else:
+                assert launches <= 2 and reported == 1
+    finally:
+        spblas.set_option("spmm_col_blocks", -1)
+        spblas.destroy(A)
