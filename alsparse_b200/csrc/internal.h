@@ -65,8 +65,8 @@ cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_
 // ... on a stream of its own, beside what is queued on `st` (which must not touch `dst`); later work on `st` waits for it.
 cudaError_t copy_to_device_beside(void *dst, const void *src, size_t bytes, cudaStream_t st);
 // Device -> host, any number of arrays one behind the other: the constructor enqueues what fits the page-locked ring
-// behind the work on `st`, finish() moves the rest and returns when every destination is complete.  Downloads of one
-// device run one after the other (a live object holds the ring), so a thread has at most one at a time.
+// behind the work on `st`, finish() moves the rest and returns when every destination is complete.  A live object holds
+// the ring; one made meanwhile copies without it.
 struct Ring;
 class Download {
   public:

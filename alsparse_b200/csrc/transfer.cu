@@ -86,6 +86,9 @@ void host_copy(void *dst, const void *src, size_t bytes) {
 // One ring per direction and device, made on first use and kept (2 x 16 MB page-locked per device in use).  A transfer
 // holds its ring's lock; an upload returns once its last piece is in the ring (the source may go away), a download
 // once everything is in host memory.
+//
+// Nobody waits here for another caller: whoever finds the ring taken, or its chunks full of copies queued on another
+// stream behind who knows what, copies directly, as slow as CUDA moves pageable memory and as independent.
 
 constexpr int kRingChunks = 4;
 constexpr size_t kRingChunkBytes = (size_t)4 << 20;
@@ -97,6 +100,7 @@ struct Ring {
     bool ready = false;
     char *buf[kRingChunks] = {};
     cudaEvent_t ev[kRingChunks] = {};
+    unsigned long long by[kRingChunks] = {};  // number of the stream whose copy `ev` stands behind
     int next = 0;
     cudaStream_t side = nullptr;  // copy_to_device_beside
     cudaEvent_t side_done = nullptr;
@@ -133,6 +137,14 @@ bool being_captured(cudaStream_t st) {
     return true;
 }
 
+// Its number, which no other stream ever has; false while it is being captured.
+static bool stream_number(cudaStream_t st, unsigned long long *number) {
+    if (being_captured(st)) return false;  // (a graph runs where it is launched)
+    if (cudaStreamGetId(st, number) == cudaSuccess) return true;
+    (void)cudaGetLastError();
+    return false;
+}
+
 bool page_locked(const void *p) {
     cudaPointerAttributes at;
     if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
@@ -145,20 +157,30 @@ bool page_locked(const void *p) {
 cudaError_t copy_to_device(void *dst, const void *src, size_t bytes, cudaStream_t st) {
     if (bytes == 0) return cudaSuccess;
     Ring *ring = nullptr;
-    if (bytes >= kRingMinBytes && !page_locked(src) && !being_captured(st)) {
+    unsigned long long number = 0;
+    if (bytes >= kRingMinBytes && !page_locked(src) && stream_number(st, &number)) {
         cudaError_t e = ring_of_current_device(g_up, &ring);
         if (e != cudaSuccess) return e;
     }
     if (!ring) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
-    std::lock_guard<std::mutex> lock(ring->mu);
-    if (!ring_ready(*ring)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    std::unique_lock<std::mutex> lock(ring->mu, std::try_to_lock);
+    if (!lock.owns_lock() || !ring_ready(*ring)) return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
     for (size_t off = 0; off < bytes; off += kRingChunkBytes) {
         const size_t n = std::min(kRingChunkBytes, bytes - off);
-        const int k = ring->next;
+        int k = -1;
+        for (int i = 0; i < kRingChunks && k < 0; i++) {  // the next chunk whose copy is done, or queued in front of ours
+            const int at = (ring->next + i) % kRingChunks;
+            if (ring->by[at] == number || cudaEventQuery(ring->ev[at]) == cudaSuccess) k = at;
+            else (void)cudaGetLastError();
+        }
+        if (k < 0)
+            return cudaMemcpyAsync(static_cast<char *>(dst) + off, static_cast<const char *>(src) + off, bytes - off,
+                                   cudaMemcpyHostToDevice, st);
         ring->next = (k + 1) % kRingChunks;
         cudaError_t e = cudaEventSynchronize(ring->ev[k]);  // the copy that used this chunk last is done
         if (e != cudaSuccess) return e;
         host_copy(ring->buf[k], static_cast<const char *>(src) + off, n);
+        ring->by[k] = number;
         e = cudaMemcpyAsync(static_cast<char *>(dst) + off, ring->buf[k], n, cudaMemcpyHostToDevice, st);
         if (e == cudaSuccess) e = cudaEventRecord(ring->ev[k], st);
         if (e != cudaSuccess) return e;
@@ -174,7 +196,8 @@ cudaError_t copy_to_device_beside(void *dst, const void *src, size_t bytes, cuda
     cudaStream_t side = nullptr;
     cudaEvent_t done = nullptr;
     {
-        std::lock_guard<std::mutex> lock(ring->mu);
+        std::unique_lock<std::mutex> lock(ring->mu, std::try_to_lock);
+        if (!lock.owns_lock()) return copy_to_device(dst, src, bytes, st);
         if (!ring->side_done) {
             e = cudaStreamCreateWithFlags(&ring->side, cudaStreamNonBlocking);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ring->side_done, cudaEventDisableTiming);
@@ -216,7 +239,7 @@ Download::Download(std::initializer_list<Piece> pieces, cudaStream_t st) : st_(s
     Ring *ring = nullptr;
     error_ = ring_of_current_device(g_down, &ring);
     if (error_ != cudaSuccess || !ring) return;
-    ring->mu.lock();
+    if (!ring->mu.try_lock()) return;  // copied by finish()
     if (!ring_ready(*ring)) {
         ring->mu.unlock();
         return;
@@ -331,13 +354,6 @@ bool device_cache_trim() {
     }
     for (const CacheBlock &b : out) cache_free(b);
     return !out.empty();
-}
-
-static bool stream_number(cudaStream_t st, unsigned long long *number) {
-    if (being_captured(st)) return false;  // (a graph runs where it is launched)
-    if (cudaStreamGetId(st, number) == cudaSuccess) return true;
-    (void)cudaGetLastError();
-    return false;
 }
 
 void BlockUse::add(cudaStream_t st) {

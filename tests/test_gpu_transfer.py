@@ -1,6 +1,7 @@
 """Page-locked rings and recycled device blocks: what else the process is doing meanwhile."""
 import ctypes as C
 import threading
+import time
 
 import numpy as np
 import pytest
@@ -132,3 +133,42 @@ def test_memory_of_a_destroyed_handle_is_not_handed_out_under_its_products():
         spblas.destroy(A)
         A = assemble(v)
     spblas.destroy(A)
+
+
+@pytest.mark.parametrize("way", ["up", "down"])
+def test_copies_do_not_wait_for_another_thread(way):
+    """A product behind a long queue on one stream, and one with vectors as large on an idle stream from another thread."""
+    m = synth.poisson("d", 7, 900000, 3300000, 3.0)  # x 26 MB, more than a ring holds; y 7 MB
+    x = synth.vector("d", 7, 1, m.cols)
+    dx = torch.from_numpy(x).cuda()
+    streams, handles = [torch.cuda.Stream() for _ in range(2)], [make_handle("d", m) for _ in range(2)]
+    ys = [np.zeros(m.nrows) if way == "down" else torch.zeros(m.nrows, dtype=torch.float64, device="cuda") for _ in range(2)]
+
+    def call(i):
+        assert spblas.mv("d", 0, 1.0, handles[i], spblas.descr(), dx if way == "down" else x, 0.0, ys[i]) == capi.SUCCESS
+
+    try:
+        for i in range(2):  # (staging buffers and, once, the answer)
+            spblas.set_stream(streams[i].cuda_stream)
+            call(i)
+            torch.cuda.synchronize()
+        want = ys[0].copy() if way == "down" else ys[0].clone()
+        with torch.cuda.stream(streams[0]):
+            torch.cuda._sleep(2_000_000_000)  # about a second
+            queued = torch.cuda.Event()
+            queued.record()
+        spblas.set_stream(streams[0].cuda_stream)  # (read when a call begins)
+        first = threading.Thread(target=call, args=(0,))
+        first.start()
+        time.sleep(0.2)
+        spblas.set_stream(streams[1].cuda_stream)
+        call(1)
+        assert not queued.query(), "the call waited for the other thread's"
+        first.join()
+    finally:
+        spblas.set_stream(None)
+    torch.cuda.synchronize()
+    for y in ys:
+        assert (y == want).all()
+    for A in handles:
+        spblas.destroy(A)
