@@ -118,6 +118,7 @@ def prototypes():
     p["alphasparse_cuda_kernel_status"] = (C.c_int, [_H, C.POINTER(C.c_int), C.c_int])
     p["alphasparse_cuda_profile_kernel"] = (C.c_int, [_H, C.c_int])
     p["alphasparse_cuda_kernel_ms"] = (C.c_int, [_H, C.POINTER(C.c_float)])
+    p["alphasparse_cuda_release_cached_memory"] = (C.c_int, [])
     p["alphasparse_cuda_debug_fail_alloc"] = (C.c_int, [C.c_int64])
     p["alphasparse_cuda_launch_count"] = (C.c_int64, [])
     p["alphasparse_cuda_last_error"] = (C.c_char_p, [])

@@ -336,9 +336,9 @@ static alphasparse_status_t coo_to_csr_keyed(int64_t rows, int64_t cols, int64_t
     int *d_ri, *d_ci;
     T *d_v;
     unsigned long long *d_bad;
-    TRY(device_block_take(layout(nullptr, &d_ri, &d_ci, &d_v, &d_bad).second, st, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    TRY(device_block_take(layout(nullptr, &d_ri, &d_ci, &d_v, &d_bad).second, st, false, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
     const SortScratch<K> sort = layout(scratch.b.p, &d_ri, &d_ci, &d_v, &d_bad).first;
-    TRY(device_block_take(adopt_block_bytes(sizeof(T), rows, nnz), st, &result.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+    TRY(device_block_take(adopt_block_bytes(sizeof(T), rows, nnz), st, true, &result.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
     int *d_ptr, *d_col;
     T *d_val;
     adopt_block_layout(result.b.p, rows, nnz, &d_ptr, &d_col, &d_val);
@@ -452,7 +452,7 @@ alphasparse_status_t transpose_csr_device(const DeviceCtx *c, int **out_ptr, int
     if (nnz > 0) {
         Carve need(nullptr);
         (void)SortScratch<unsigned>(need, nnz);
-        TRY(device_block_take(need.used, st, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+        TRY(device_block_take(need.used, st, false, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
         Carve have(scratch.b.p);
         const SortScratch<unsigned> sort(have, nnz);
         TRY(cudaMemcpyAsync(sort.keys[0], c->d_col, sizeof(int) * n, cudaMemcpyDeviceToDevice, st),
@@ -652,7 +652,7 @@ alphasparse_status_t derive_csr_device(const DeviceCtx *c, int type, int upper, 
     if (m > 0) {
         Carve need(nullptr);
         (void)SortScratch<unsigned long long>(need, m);
-        TRY(device_block_take(need.used, st, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
+        TRY(device_block_take(need.used, st, false, &scratch.b), ALPHA_SPARSE_STATUS_ALLOC_FAILED);
         Carve have(scratch.b.p);
         const SortScratch<unsigned long long> sort(have, m);
         const int bits = bits_for(rows);  // square: rows == cols

@@ -298,7 +298,7 @@ alphasparse_status_t ctx_adopt_block(int datatype, int64_t rows, int64_t cols, i
     c->device = c->block.device, c->datatype = datatype, c->rows = rows, c->cols = cols, c->nnz = nnz;
     c->d_row_ptr = reinterpret_cast<int *>(p), c->d_col = reinterpret_cast<int *>(p + l.col), c->d_val = p + l.val;
     c->d_status = reinterpret_cast<int *>(p + l.status), c->d_stats = reinterpret_cast<unsigned long long *>(p + l.stats);
-    c->device_bytes = (int64_t)l.bytes;
+    c->device_bytes = (int64_t)c->block.bytes;
     block_used(c, current_stream());
     cudaError_t e = cudaMemsetAsync(c->d_status, 0, sizeof(int), current_stream());
     alphasparse_status_t s = ALPHA_SPARSE_STATUS_EXECUTION_FAILED;
@@ -1745,6 +1745,12 @@ alphasparse_status_t alphasparse_cuda_kernel_ms(const alphasparse_matrix_t A, fl
     ASB_CUDA_OR(cudaEventElapsedTime(ms, c->ev_start, c->ev_stop), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
+alphasparse_status_t alphasparse_cuda_release_cached_memory(void) {
+    device_cache_trim();
+    host_pools_trim();
+    return ALPHA_SPARSE_STATUS_SUCCESS;
+}
+
 alphasparse_status_t alphasparse_cuda_debug_fail_alloc(int64_t nth) {
     g_fail_alloc_in.store(nth > 0 ? nth : 0, std::memory_order_relaxed);
     return ALPHA_SPARSE_STATUS_SUCCESS;

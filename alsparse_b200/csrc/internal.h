@@ -113,9 +113,12 @@ struct BlockUse {
     unsigned long long stream = 0;  // its number: never used twice, as an address may be
     void add(cudaStream_t st);      // work is about to be queued on `st`
 };
-cudaError_t device_block_take(size_t bytes, cudaStream_t st, DeviceBlock *out);  // for use on `st` first of all
+// For use on `st` first of all.  A recycled block may be up to twice as large as asked for, one that is `kept` with a
+// handle up to a quarter larger.
+cudaError_t device_block_take(size_t bytes, cudaStream_t st, bool kept, DeviceBlock *out);
 void device_block_give(DeviceBlock *b, const BlockUse &use);
 bool device_cache_trim();                // gives everything cached back to CUDA; true if there was anything
+void host_pools_trim();                  // the same for the page-locked memory that no call is using
 bool device_alloc_denied();              // counts an allocation for alphasparse_cuda_debug_fail_alloc; true: it is to fail
 
 // Every device allocation of the library goes through here: cudaMalloc, except that a test can ask

@@ -314,6 +314,27 @@ void host_block_give(const HostBlock &b) {
     g_host_block_taken[b.index] = false;
 }
 
+void host_pools_trim() {
+    for (Ring *rings : {g_up, g_down})
+        for (int d = 0; d < kRingDevices; d++) {
+            Ring &r = rings[d];
+            std::unique_lock<std::mutex> lock(r.mu, std::try_to_lock);
+            if (!lock.owns_lock() || !r.ready) continue;
+            for (int k = 0; k < kRingChunks; k++) {  // (its copies may still be queued)
+                cudaError_t e = cudaEventSynchronize(r.ev[k]);
+                if (e == cudaSuccess) e = cudaFreeHost(r.buf[k]);
+                if (e == cudaSuccess) r.buf[k] = nullptr, r.ready = false;
+                else (void)cudaGetLastError();
+            }
+        }
+    std::lock_guard<std::mutex> lock(g_host_block_mu);
+    for (int k = 0; k < kHostBlocks; k++) {
+        if (g_host_block_taken[k] || !g_host_block[k].p) continue;
+        if (cudaFreeHost(g_host_block[k].p) != cudaSuccess) (void)cudaGetLastError();
+        g_host_block[k].p = nullptr;
+    }
+}
+
 // ---- device blocks of assembled matrices ---------------------------------------------------------------
 //
 // Converting triples needs scratch for the sort and one block for the resulting arrays.  A program that assembles its
@@ -363,7 +384,7 @@ void BlockUse::add(cudaStream_t st) {
     else where = kOneStream, stream = number;
 }
 
-cudaError_t device_block_take(size_t bytes, cudaStream_t st, DeviceBlock *out) {
+cudaError_t device_block_take(size_t bytes, cudaStream_t st, bool kept, DeviceBlock *out) {
     *out = DeviceBlock{};
     const size_t want = (std::max<size_t>(bytes, 1) + kCacheGrain - 1) / kCacheGrain * kCacheGrain;
     int dev = 0;
@@ -372,13 +393,14 @@ cudaError_t device_block_take(size_t bytes, cudaStream_t st, DeviceBlock *out) {
     if (device_alloc_denied()) return cudaErrorMemoryAllocation;
     unsigned long long number = 0;
     const bool numbered = stream_number(st, &number);
+    const size_t most = kept ? want + want / 4 : 2 * want;
     bool wait = false;
     {
         std::lock_guard<std::mutex> lock(g_cache_mu);
         size_t best = g_cache.size();
         for (size_t i = 0; i < g_cache.size(); i++) {
             const CacheBlock &c = g_cache[i];
-            if (c.device != dev || c.bytes < want || c.bytes > 2 * want) continue;
+            if (c.device != dev || c.bytes < want || c.bytes > most) continue;
             if (c.use.where != BlockUse::kNowhere && !(numbered && c.use.stream == number)) continue;
             if (best == g_cache.size() || c.bytes < g_cache[best].bytes) best = i;
         }

@@ -224,6 +224,11 @@ def kernel_ms(A):
     return ms.value
 
 
+def release_cached_memory():
+    """alphasparse_cuda_release_cached_memory: what the library keeps for later calls goes back to CUDA."""
+    return capi.load().alphasparse_cuda_release_cached_memory()
+
+
 def csrmv_noalloc(rows, cols, nnz, alpha, d_row_ptr, d_col_indx, d_values, d_x, beta, d_y):
     """alphasparse_cuda_d_csrmv_noalloc: double-precision SpMV on device arrays that never allocates
     (scratch lives in a fixed 4 MiB array inside the library; rows + nnz <= 375,802,112)."""

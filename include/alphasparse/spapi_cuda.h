@@ -210,6 +210,15 @@ alphasparse_status_t alphasparse_cuda_kernel_status(const alphasparse_matrix_t A
 alphasparse_status_t alphasparse_cuda_profile_kernel(const alphasparse_matrix_t A, int enable);
 alphasparse_status_t alphasparse_cuda_kernel_ms(const alphasparse_matrix_t A, float *ms);
 
+/* Returns to CUDA what the library keeps between calls and no other call is using at the moment:
+ *   - device blocks of converted matrices and of their sorting, for the next conversion: at most 512 MB over
+ *     all devices, no block above 256 MB (they also go back when an allocation of the library's own fails);
+ *   - two page-locked rings of 16 MB for every device that has copied pageable arrays of 64 KB or more;
+ *   - up to 4 MB of page-locked blocks for small host vectors.
+ * For programs whose other parts need the memory, and before cudaDeviceReset, which would take it away under the
+ * library.  Later calls allocate afresh.  Handles keep what is theirs (device_bytes above). */
+alphasparse_status_t alphasparse_cuda_release_cached_memory(void);
+
 /* Test aid: makes the nth device allocation the library performs from now on fail as if the device
  * were out of memory (0 cancels).  The failing call returns ALPHA_SPARSE_STATUS_ALLOC_FAILED and
  * releases whatever it had already allocated. */

@@ -172,3 +172,34 @@ def test_copies_do_not_wait_for_another_thread(way):
         assert (y == want).all()
     for A in handles:
         spblas.destroy(A)
+
+
+def test_kept_memory_is_reported_and_given_back():
+    """What conversions leave in the cache can be had back, and a handle reports the block it really holds."""
+    def assemble(nnz):
+        rng = np.random.default_rng(nnz)
+        ri, ci = rng.integers(50000, size=nnz, dtype=np.int32), rng.integers(50000, size=nnz, dtype=np.int32)
+        st, coo = spblas.create_coo("d", capi.BASE_ZERO, 50000, 50000, nnz, ri, ci, np.ones(nnz))
+        st2, A = spblas.convert_csr(coo)
+        assert st == st2 == capi.SUCCESS, spblas.last_error()
+        spblas.destroy(coo)
+        return A
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    spblas.destroy(assemble(3000000))  # (kernels loaded)
+    assert spblas.release_cached_memory() == capi.SUCCESS
+    base = free()
+    spblas.destroy(assemble(3000000))
+    assert free() < base - (30 << 20)  # kept for the next conversion
+    A = assemble(1700000)  # its arrays take a little more than half of the block that lies there
+    spblas.release_cached_memory()
+    held, reported = base - free(), spblas.mat_info(A)[1].device_bytes
+    assert abs(held - reported) <= 6 << 20  # CUDA hands memory out in pieces of 2 MB
+    assert reported <= 1.3 * 1700000 * 12 + (1 << 20)
+    check_mv("d", synth.poisson("d", 6, 300000, 300000, 9.0), 1.5, 0.5)  # rings made anew
+    spblas.destroy(A)
+    spblas.release_cached_memory()
+    assert abs(base - free()) <= 2 << 20
