@@ -637,13 +637,18 @@ void spmm_segments_destroy(SpmmSegments &s) {
     s = SpmmSegments{};
 }
 
-// Built at the first product of a handle whose rows are uneven (the rule of spmm_split_ensure: even rows need no table).
+// Rows of such lengths that segments of whole rows would not be of equal work.
+static bool spmm_uneven(const DeviceCtx *ctx) {
+    return option(kOptSpmmSplitMin) > 0 && ctx->max_row_nnz > kStreamWhole && (double)ctx->max_row_nnz > 8.0 * ctx->mean_row_nnz;
+}
+
+// Built at the first product of a handle whose rows are uneven (even rows need no table).
 // Segments of 64 to 256 items, enough of them to keep every warp of the chip (about 5,000) busy twice.
 static alphasparse_status_t spmm_segments_ensure(DeviceCtx *ctx, cudaStream_t st) {
     SpmmSegments &sp = ctx->segments;
     if (sp.state != 0) return ALPHA_SPARSE_STATUS_SUCCESS;
     const int64_t most = std::max<int64_t>(64, std::min<int64_t>(256, option(kOptSpmmSplitChunk)));
-    if (option(kOptSpmmSplitMin) <= 0 || ctx->max_row_nnz <= kStreamWhole || (double)ctx->max_row_nnz <= 8.0 * ctx->mean_row_nnz) {
+    if (!spmm_uneven(ctx)) {
         sp.state = 1;
         return ALPHA_SPARSE_STATUS_SUCCESS;
     }
@@ -764,9 +769,54 @@ static int spmm_pick_blocks(const DeviceCtx *ctx) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(blocks, 64));
 }
 
-// One pass per column block (option spmm_col_blocks): spmm_row_kernel over the part of every row inside the block.
+// Which of the two kernels multiplies: a lane group per row (spmm_row_kernel: 32 / LPR rows end at once, nothing is
+// fetched ahead) or a warp walking the elements (spmm_stream_kernel: ending a row takes the whole warp some 200
+// instructions and, with beta != 0, a wait for Y, but X rows are requested ahead).  So rows of few elements go to the
+// former, and the more so the fewer lanes a row takes, where Y is read, and where X rows come quickly because neighbouring
+// rows share them (`banded`).  Measured (B200, row / stream kernel, us): diagonal of 262,144 rows x 12 fp32 columns, beta
+// != 0 12.4 / 53.9; 2^20 rows of 5 x 12 94 / 216, x 64 359 / 384, x 128 718 / 711; 2^20 rows of 12 x 16, banded 122 / 187; 2^19
+// rows of 20 x 12 172 / 153, banded 105 / 140; 262,144 rows of 27 x 24 145 / 109, x 64 261 / 219.  The limits below are mean row
+// lengths at which the two were level, from 10,900 pairs over 2^10 to 2^22 rows, 1 to 160 elements, 5 to 256 columns and both
+// precisions; a rule that always knew would be 1.1 % faster over those.
+//
+// With fewer rows than fill the chip a few times over, what counts is the longest row: the row kernel walks it four
+// elements at a time, 0.24 us each, while the stream kernel takes 6-8 us however long its rows.  (2^13 rows of 8 +- 3 x 12 fp32
+// columns 13 / 7, all of 8 7 / 11.)  That also bounds what an uneven matrix may have: its longest row has to be done in the
+// time of the others (2^20 rows of 1 and one of 100 x 12 82 / 176, one of 400 186 / 177; 262,144 rows and one of 400 119 / 48),
+// and wider blocks are worth it only where the stream kernel would wait for Y (2^20 x 24 and one of 100 130 / 196, beta = 0
+// 119 / 113).
+//
+// An odd number of columns below 32 in single precision fills its one slice of 32 lanes: the limits of {4, 32} are those of
+// more columns, whose last slice is nearly empty (2^20 rows of 1 x 31, beta = 0 225 / 114, x 33 275 / 230).
+static bool spmm_row_by_row(const DeviceCtx *ctx, int lane_bytes, int lanes, int columns, bool has_beta) {
+    struct Limit {
+        int lane_bytes, lanes;
+        float mean[2][2];  // [banded][beta != 0]
+        int longest;       // of up to kRowsFew rows
+    };
+    static const Limit limits[] = {
+        {16, 4, {{9.f, 12.5f}, {15.f, 30.f}}, 11}, {16, 8, {{5.f, 9.f}, {10.f, 15.f}}, 15},
+        {16, 16, {{0.7f, 5.f}, {3.f, 10.f}}, 21},  {16, 32, {{0.8f, 5.f}, {0.5f, 0.9f}}, 24},
+        {8, 8, {{8.f, 12.f}, {15.f, 40.f}}, 15},   {8, 16, {{0.7f, 10.f}, {7.f, 27.f}}, 21},
+        {8, 32, {{0.9f, 28.f}, {0.7f, 0.8f}}, 44}, {4, 16, {{160.f, 40.f}, {30.f, 160.f}}, 24},
+        {4, 32, {{7.f, 30.f}, {1.f, 15.f}}, 44},
+    };
+    constexpr int64_t kRowsOneWave = 148 * 32, kRowsFew = 40000;
+    const Limit *l = std::find_if(std::begin(limits), std::end(limits),
+                                  [&](const Limit &c) { return c.lane_bytes == lane_bytes && c.lanes == lanes; });
+    if (l == std::end(limits)) l = limits;  // (few lanes of few bytes: blocks of at most 32 bytes, asked for by option)
+    float mean = l->mean[ctx->shifted_rows >= 0.5][has_beta];
+    if (lane_bytes == 4 && columns < 32 && lanes == 32 && !has_beta) mean = std::min(mean, 0.9f);
+    if (spmm_uneven(ctx))
+        return (has_beta || lanes == 4) && 20000 * ctx->max_row_nnz <= ctx->rows + ctx->nnz && ctx->mean_row_nnz <= 0.5 * mean;
+    if (ctx->rows <= kRowsFew) return ctx->max_row_nnz <= (ctx->rows <= kRowsOneWave ? std::max(8, l->longest / 3) : l->longest);
+    return ctx->mean_row_nnz <= mean;
+}
+
+// spmm_row_kernel over whole rows, or (option spmm_col_blocks) in one pass per column block over the part of every row
+// inside the block.
 template <typename T, int VEC, int LPR>
-static void launch_row_blocks(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
+static void launch_row_groups(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
                               int ldy, cudaStream_t st, const RowWindow *w) {
     constexpr int rows_per_block = 8 * (32 / LPR);
     // A window is the same kernel on a slice: offsets are absolute, so shifting the offset arrays and Y
@@ -775,8 +825,10 @@ static void launch_row_blocks(DeviceCtx *ctx, T alpha, const T *X, int columns, 
     const unsigned blocks = (unsigned)((rows + rows_per_block - 1) / rows_per_block);
     const T *val = static_cast<const T *>(ctx->d_val);
     Y += first * (int64_t)ldy;
-    for (int p = 0; p < ctx->spmm.blocks; p++) {
-        const int *lo = ctx->spmm.d_split + (size_t)p * ctx->rows + first, *hi = lo + ctx->rows;
+    const int passes = ctx->spmm.d_split ? ctx->spmm.blocks : 1;
+    for (int p = 0; p < passes; p++) {
+        const int *lo = ctx->spmm.d_split ? ctx->spmm.d_split + (size_t)p * ctx->rows + first : ctx->d_row_ptr + first;
+        const int *hi = ctx->spmm.d_split ? lo + ctx->rows : lo + 1;
         // the first pass applies beta, the later ones add to what is there
         const T b = p == 0 ? beta : T(1);
         if (b == T(0))
@@ -786,19 +838,23 @@ static void launch_row_blocks(DeviceCtx *ctx, T alpha, const T *X, int columns, 
             spmm_row_kernel<T, VEC, LPR, true><<<blocks, 256, 0, st>>>(
                 (int)rows, lo, hi, ctx->d_col, val, X, columns, ldx, Y, ldy, alpha, b);
     }
-    count_launch(ctx->spmm.blocks);
+    count_launch(passes);
 }
 
 template <typename T, int VEC, int LPR>
-static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
-                       int ldy, cudaStream_t st, const RowWindow *w, T *part) {
+static alphasparse_status_t launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
+                                       int ldy, cudaStream_t st, const RowWindow *w) {
+    T *part = nullptr;
+    if (ctx->spmm.d_split || spmm_row_by_row(ctx, VEC * (int)sizeof(T), LPR, columns, beta != T(0))) {
+        if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
+        launch_row_groups<T, VEC, LPR>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+        if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
+        return ALPHA_SPARSE_STATUS_SUCCESS;
+    }
+    const alphasparse_status_t s = spmm_segments_prepare<T>(ctx, columns, st, &part);
+    if (s != ALPHA_SPARSE_STATUS_SUCCESS) return s;
     SpmmSegments &sp = ctx->segments;
     if (ctx->profile) cudaEventRecord(ctx->ev_start, st);
-    if (ctx->spmm.d_split) {
-        launch_row_blocks<T, VEC, LPR>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
-        if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
-        return;
-    }
     const int row0 = (int)(w ? w->begin : 0), row1 = (int)(w ? w->begin + w->count : ctx->rows);
     StreamSegments sg{};
     sg.row0 = row0, sg.row1 = row1;
@@ -840,11 +896,12 @@ static void launch_row(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx
         }
     }
     if (ctx->profile) cudaEventRecord(ctx->ev_stop, st);
+    return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
 template <typename T, int VEC>
-static void launch_row_lanes(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
-                             int ldy, cudaStream_t st, const RowWindow *w, T *part) {
+static alphasparse_status_t launch_row_lanes(DeviceCtx *ctx, T alpha, const T *X, int columns, int ldx, T beta, T *Y,
+                                             int ldy, cudaStream_t st, const RowWindow *w) {
     // smallest group (4 .. 32 lanes) whose lanes cover the dense columns in one pass, if any
     const int need = (columns + VEC - 1) / VEC;
     // An X beyond L2 (126 MB) with unstructured columns is read in slices of 256 bytes a row: the part of X in use is half
@@ -853,10 +910,11 @@ static void launch_row_lanes(DeviceCtx *ctx, T alpha, const T *X, int columns, i
     // (50,000 rows x 128 fp64 columns 139 -> 158), neighbouring rows share X rows (stencil 78^3 x 128 fp64 933 -> 1042) or
     // lanes hold less than 16 bytes (200,000 rows x 127 fp32 columns 603 -> 877).
     const bool sliced = VEC * sizeof(T) == 16 && ctx->shifted_rows < 0.5 && sizeof(T) * (size_t)ctx->cols * columns > (126u << 20);
-    if (need <= 4) launch_row<T, VEC, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
-    else if (need <= 8) launch_row<T, VEC, 8>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
-    else if (need <= 16 || sliced) launch_row<T, VEC, 16>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
-    else launch_row<T, VEC, 32>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+    if (need <= 4) return launch_row<T, VEC, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+    if (need <= 8) return launch_row<T, VEC, 8>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+    if (need <= 16 || (sliced && !spmm_row_by_row(ctx, VEC * (int)sizeof(T), 32, columns, beta != T(0))))
+        return launch_row<T, VEC, 16>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+    return launch_row<T, VEC, 32>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
 }
 
 template <typename T, int LANES, int KC, bool ALIGNED>
@@ -934,7 +992,6 @@ alphasparse_status_t launch_spmm_row(DeviceCtx *ctx, T alpha, const T *X, int co
     if (ctx->rows == 0 || columns <= 0 || (w && w->count <= 0)) return ALPHA_SPARSE_STATUS_SUCCESS;
     block_used(ctx, st);
     const bool narrow = (size_t)columns * sizeof(T) <= 32 && option(kOptSpmmNarrow);
-    T *part = nullptr;
     alphasparse_status_t bs;
     if (narrow) {
         bs = spmm_split_prepare(ctx, sizeof(T), columns, st);
@@ -944,7 +1001,6 @@ alphasparse_status_t launch_spmm_row(DeviceCtx *ctx, T alpha, const T *X, int co
         return ALPHA_SPARSE_STATUS_SUCCESS;
     }
     bs = col_blocks_ensure(ctx, ctx->spmm, spmm_pick_blocks(ctx), st);
-    if (bs == ALPHA_SPARSE_STATUS_SUCCESS && !ctx->spmm.d_split) bs = spmm_segments_prepare<T>(ctx, columns, st, &part);
     if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
     auto fits = [&](int vec) {
         const uintptr_t mask = (uintptr_t)(vec * sizeof(T) - 1);
@@ -953,13 +1009,14 @@ alphasparse_status_t launch_spmm_row(DeviceCtx *ctx, T alpha, const T *X, int co
     };
     // Widest 16-byte pack the shapes and alignments allow.
     if constexpr (sizeof(T) == 4) {
-        if (fits(4)) launch_row_lanes<T, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
-        else if (fits(2)) launch_row_lanes<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
-        else launch_row_lanes<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+        if (fits(4)) bs = launch_row_lanes<T, 4>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+        else if (fits(2)) bs = launch_row_lanes<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+        else bs = launch_row_lanes<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
     } else {
-        if (fits(2)) launch_row_lanes<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
-        else launch_row_lanes<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w, part);
+        if (fits(2)) bs = launch_row_lanes<T, 2>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
+        else bs = launch_row_lanes<T, 1>(ctx, alpha, X, columns, ldx, beta, Y, ldy, st, w);
     }
+    if (bs != ALPHA_SPARSE_STATUS_SUCCESS) return bs;
     ASB_CUDA_OR(cudaGetLastError(), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
