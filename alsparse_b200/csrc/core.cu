@@ -859,6 +859,17 @@ static alphasparse_status_t ensure_pipe(DeviceCtx *c) {
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
+// The end of a call with host operands: waits for `st`, and reports a kernel whose bounded wait ran out.
+static alphasparse_status_t wait_and_report(DeviceCtx *c, cudaStream_t st) {
+    int kernel_status = 0;
+    ASB_CUDA_OR(cudaMemcpyAsync(&kernel_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, st),
+                ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    ASB_CUDA_OR(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    if (kernel_status == 0) return ALPHA_SPARSE_STATUS_SUCCESS;
+    (void)cudaMemsetAsync(c->d_status, 0, sizeof(int), st);  // reported once: later calls start clean
+    return ALPHA_SPARSE_STATUS_EXECUTION_FAILED;
+}
+
 template <typename T>
 static alphasparse_status_t mv_host_pipelined(DeviceCtx *c, T alpha, const T *x, bool x_dev, T beta, T *y,
                                               cudaStream_t st) {
@@ -1054,17 +1065,7 @@ static alphasparse_status_t mv_on_ctx(DeviceCtx *c, T alpha, const T *x, T beta,
         if (s != ALPHA_SPARSE_STATUS_SUCCESS) return s;
         if (!y_dev) ASB_CUDA_OR(copy_to_host(y, dy, sizeof(T) * (size_t)c->rows, st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     }
-    if (!y_dev || !x_dev) {
-        // a synchronous call can also report a kernel whose bounded wait ran out
-        int kernel_status = 0;
-        ASB_CUDA_OR(cudaMemcpyAsync(&kernel_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, st),
-                    ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-        ASB_CUDA_OR(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-        if (kernel_status != 0) {  // reported once: later calls start clean
-            (void)cudaMemsetAsync(c->d_status, 0, sizeof(int), st);
-            return ALPHA_SPARSE_STATUS_EXECUTION_FAILED;
-        }
-    }
+    if (!y_dev || !x_dev) return wait_and_report(c, st);
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 
@@ -1206,8 +1207,10 @@ static alphasparse_status_t mm_on_ctx(DeviceCtx *c, alphasparse_layout_t layout,
     if (!y_dev)
         ASB_CUDA_OR(cudaMemcpyAsync(y, dy, ybytes, cudaMemcpyDeviceToHost, st),
                     ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
-    if (!y_dev || !x_dev)
-        ASB_CUDA_OR(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
+    if (y_dev && x_dev) return ALPHA_SPARSE_STATUS_SUCCESS;
+    // (the row-major kernels have nothing to wait for)
+    if (!row_major && c->algorithm == ALPHA_SPARSE_CUDA_ALG_ROWTILE) return wait_and_report(c, st);
+    ASB_CUDA_OR(cudaStreamSynchronize(st), ALPHA_SPARSE_STATUS_EXECUTION_FAILED);
     return ALPHA_SPARSE_STATUS_SUCCESS;
 }
 

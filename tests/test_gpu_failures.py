@@ -10,7 +10,7 @@ import torch
 
 import oracle
 from alsparse_b200 import capi, multi, spblas, synth
-from gpu_util import make_handle
+from gpu_util import _DeviceArray, make_handle
 from helpers import assert_rows_close, row_scale
 
 pytestmark = pytest.mark.gpu
@@ -85,3 +85,23 @@ def test_concurrent_callers_on_one_handle():
         y_ref = oracle.gemv("s", m.rows_start, m.rows_end, m.col, m.val, 1.0, xs[i], 0.0, np.zeros(m.nrows, np.float32))
         assert_rows_close("s", ys[i], y_ref, row_scale(m.ptr, m.col, m.val, xs[i], 1.0, 0.0, y_ref * 0), f"thread {i}")
     spblas.destroy(A)
+
+
+def test_a_dense_block_product_on_host_operands_reports_its_kernels():
+    """The error word is set from here: it lies behind the values of a matrix that was converted on the device."""
+    m = synth.stencil27("d", 12)
+    rows = np.repeat(np.arange(m.nrows, dtype=np.int32), np.diff(m.ptr))
+    st, coo = spblas.create_coo("d", capi.BASE_ZERO, m.nrows, m.cols, m.nnz, rows, m.col, m.val)
+    st2, A = spblas.convert_csr(coo)
+    assert st == st2 == capi.SUCCESS and spblas.mat_info(A)[1].algorithm == capi.ALG_ROWTILE
+    _, _, _, d_val = spblas.device_csr(A)
+    word = torch.as_tensor(_DeviceArray(d_val + (8 * (m.nnz + 16) + 255) // 256 * 256, 1, "<i4"), device="cuda")
+    assert spblas.kernel_status(A) == (capi.SUCCESS, 0)
+    word.fill_(2)
+    torch.cuda.synchronize()
+    assert spblas.kernel_status(A) == (capi.SUCCESS, 2)  # it is the error word
+    X, Y = np.ones(m.cols * 3), np.zeros(m.nrows * 3)
+    for want in (capi.EXECUTION_FAILED, capi.SUCCESS):  # reported once
+        assert spblas.mm("d", 0, 1.0, A, spblas.descr(), capi.COLUMN_MAJOR, X, 3, m.cols, 0.0, Y, m.nrows) == want
+    for h in (coo, A):
+        spblas.destroy(h)
