@@ -12,10 +12,12 @@ from helpers import assert_rows_close, mm_scale
 pytestmark = pytest.mark.gpu
 
 
-def banded(kind, rows, offsets):
-    """Row r holds the columns r + offsets that lie inside the matrix."""
+def banded(kind, rows, offsets, empty=None):
+    """Row r holds the columns r + offsets that lie inside the matrix; the rows of `empty` hold none."""
     col = np.arange(rows)[:, None] + np.asarray(offsets)[None, :]
     inside = (col >= 0) & (col < rows)
+    if empty is not None:
+        inside[empty] = False
     ptr = np.concatenate([[0], np.cumsum(inside.sum(1))]).astype(np.int32)
     return synth.Csr(rows, rows, 0, ptr, col[inside].astype(np.int32), synth.vector(kind, 3, 1, int(ptr[-1])))
 
@@ -23,7 +25,9 @@ def banded(kind, rows, offsets):
 @pytest.mark.parametrize("kind", ["s", "d"])
 @pytest.mark.parametrize("make", [lambda k: synth.stencil27(k, 9), lambda k: banded(k, 33, (-1, 0, 1)),
                                   lambda k: banded(k, 1000, (-40, -1, 0, 1, 40)), lambda k: banded(k, 31, range(0, 8)),
-                                  lambda k: banded(k, 4097, (-2, 5))])
+                                  lambda k: banded(k, 4097, (-2, 5)),
+                                  lambda k: banded(k, 2000, (-1, 0, 1, 7), slice(320, 400)),  # whole tiles and a part of one
+                                  lambda k: banded(k, 1001, (0, 1, 2), slice(990, None))])
 def test_tiles_and_column_groups(kind, make):
     m = make(kind)
     A = make_handle(kind, m)

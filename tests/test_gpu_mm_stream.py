@@ -156,3 +156,49 @@ def test_column_blocks_where_they_are_asked_for(longest, blocks_run):
     finally:
         spblas.set_option("spmm_col_blocks", -1)
         spblas.destroy(A)
+
+
+@pytest.mark.parametrize("shape", ["skewed", "thirty"])
+def test_rows_of_x_that_no_element_names_are_dropped(shape):
+    """The kernel reads row 0 of X behind the end of a segment: what it holds must not reach Y."""
+    lens = lengths("skewed") if shape == "skewed" else np.full(3001, 30, np.int32)
+    m = synth.from_lengths("s", 21, lens, 2500)
+    m = synth.Csr(m.nrows, m.cols + 1, 0, m.ptr, m.col + 1, m.val)  # column 0 is in no row
+    A = make_handle("s", m)
+    for columns in (12, 33, 64):
+        X = torch.rand(m.cols, columns, device="cuda")
+        Y = torch.empty(2, m.nrows, columns, device="cuda")
+        for y, worst in zip(Y, (0.0, float("nan"))):
+            X[0] = worst
+            multiply("s", A, 1.5, X, columns, columns, 0.0, y, columns)
+        torch.cuda.synchronize()
+        assert torch.equal(Y[0], Y[1])
+        X[0] = float("inf")
+        multiply("s", A, 1.5, X, columns, columns, 0.0, Y[1], columns)
+        torch.cuda.synchronize()
+        assert torch.equal(Y[0], Y[1])
+    spblas.destroy(A)
+
+
+def test_two_streams_of_one_handle_at_once():
+    """Each stream has partial sums of its own for the rows that are cut over segments."""
+    m = synth.from_lengths("d", 21, lengths("skewed"), 2500)
+    A = make_handle("d", m)
+    columns, streams = 64, [torch.cuda.Stream() for _ in range(2)]
+    xs = [torch.rand(m.cols, columns, dtype=torch.float64, device="cuda") for _ in streams]
+    ys = [torch.zeros(m.nrows, columns, dtype=torch.float64, device="cuda") for _ in streams]
+    want = [torch.zeros_like(y) for y in ys]
+    for x, y in zip(xs, want):
+        multiply("d", A, 1.0, x, columns, columns, 0.0, y, columns)
+    torch.cuda.synchronize()
+    try:
+        for _ in range(50):  # products of the two streams run side by side
+            for s, x, y in zip(streams, xs, ys):
+                spblas.set_stream(s.cuda_stream)
+                multiply("d", A, 1.0, x, columns, columns, 0.0, y, columns)
+    finally:
+        spblas.set_stream(None)
+    torch.cuda.synchronize()
+    for y, w in zip(ys, want):
+        assert torch.equal(y, w)
+    spblas.destroy(A)

@@ -424,7 +424,7 @@ def test_vector_kernel_in_column_blocks(kind):
 
 @pytest.mark.parametrize("kind", ["s", "d"])
 def test_large_coo_is_sorted_on_the_device(kind):
-    """More than 2^20 COO entries take the GPU radix-sort path of alphasparse_convert_csr; the CSR must be
+    """COO entries by the million through the GPU radix-sort path of alphasparse_convert_csr; the CSR must be
     the one the reference's conversion produces (bit-exact, duplicates kept in input order)."""
     m = synth.poisson(kind, 81, 90000, 70000, 14.0)
     assert m.nnz > 1 << 20
